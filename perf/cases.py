@@ -222,3 +222,54 @@ def run(st):
         ctx.set_device_tables(st["cos"], st["sin"])
         ctx.joint_attention_host(st["q"], st["k"], st["v"], *st["norm"], None, None, st["out"], st["p"])
     return st["out"]
+
+
+# ------------------------------------------------------------------------------------------------ in 64 bits
+def _norm_rope64(x, w_txt, w_img, cos, sin, txt, eps):
+    """[batch, tokens, heads, D] in float64: RMS norm per head, weight of the token's segment, pair rotation."""
+    x = x * torch.rsqrt((x * x).mean(-1, keepdim=True) + eps)
+    x[:, :txt] *= w_txt.double()
+    x[:, txt:] *= w_img.double()
+    even, odd = x[..., 0::2], x[..., 1::2]
+    c, s = cos.double()[None, :, None, :], sin.double()[None, :, None, :]
+    out = torch.empty_like(x)
+    out[..., 0::2] = even * c[..., 0::2] - odd * s[..., 0::2]
+    out[..., 1::2] = odd * c[..., 1::2] + even * s[..., 1::2]
+    return out
+
+
+def _attention64(q, k, v, scale, mask=None):
+    """One head: q, k, v [tokens, d] in float64, 2048 query rows at a time."""
+    out = torch.empty_like(q)
+    for r in range(0, q.shape[0], 2048):
+        scores = (q[r:r + 2048] @ k.T) * scale
+        if mask is not None:
+            scores += mask
+        out[r:r + 2048] = torch.softmax(scores, -1) @ v
+    return out
+
+
+def exact(case, seed):
+    """What ``run`` gives for these inputs, in float64 with plain torch."""
+    st = prepare(case, seed)
+    if case["kind"] == "wide":
+        return _attention64(st["q"].double(), st["k"].double(), st["v"].double(), case["channels"] ** -0.5)
+    p = st["p"]
+    b, s, h = p.batch, p.tokens, p.heads
+    if case["kind"] == "block":
+        x = st["x"].double()
+        q, k, v = ((x @ w.double().T).view(b, s, h, D) for w in st["w"][:3])
+    else:
+        q, k, v = (t.to(DEVICE) for t in (st["q"], st["k"], st["v"]))
+    norm = [w.to(DEVICE) for w in st["norm"]]
+    mask = None if st["mask"] is None else st["mask"].double()
+    out = torch.empty((b, s, h, D), dtype=torch.float64, device=DEVICE)
+    for i in range(b):
+        for j in range(h):
+            one = (slice(i, i + 1), slice(None), slice(j, j + 1))
+            qj = _norm_rope64(q[one].double(), norm[0], norm[1], st["cos"], st["sin"], p.txt_tokens, p.norm_eps)
+            kj = _norm_rope64(k[one].double(), norm[2], norm[3], st["cos"], st["sin"], p.txt_tokens, p.norm_eps)
+            out[i, :, j] = _attention64(qj[0, :, 0], kj[0, :, 0], v[one][0, :, 0].double(), D ** -0.5, mask)
+    if case["kind"] == "block":
+        return out.view(b * s, h * D) @ st["w"][3].double().T
+    return out.cpu() if case["kind"] == "host" else out
