@@ -143,7 +143,8 @@ int reserve_scratch(Ctx* c, const zdraw_cuda_attn_params* p, const Shape& s, boo
 int run_prologue(Ctx* c, cudaStream_t stream, const void* q, const void* k, const float* q_w_txt,
                  const float* q_w_img, const float* k_w_txt, const float* k_w_img, const float* rope_cos,
                  const float* rope_sin, void* q_out, void* k_out, bool out_head_major,
-                 const zdraw_cuda_attn_params* p, const Shape& s) {
+                 const zdraw_cuda_attn_params* p, const Shape& s, const void* joint_v = nullptr,
+                 const float* joint_mask = nullptr) {
   const void* ptrs[] = {q, k, q_w_txt, q_w_img, k_w_txt, k_w_img, rope_cos, rope_sin, q_out, k_out};
   for (const void* x : ptrs) {
     if (!x) return fail(c, ZDRAW_CUDA_E_ARG, "null pointer given to the prologue");
@@ -169,19 +170,39 @@ int run_prologue(Ctx* c, cudaStream_t stream, const void* q, const void* k, cons
   a.rope_batch_stride = static_cast<long long>(p->rope_batch_stride);
   a.q_out = q_out;
   a.k_out = k_out;
+  // The joint call's launch also casts an f32 V and writes the key mask's tile lists (reserved scratch).
+  if (joint_v != nullptr && p->in_dtype == ZDRAW_DTYPE_F32) {
+    a.v = static_cast<const float*>(joint_v);
+    a.ld_v = s.ld_v;
+    a.v_out = c->v16.p;
+  }
+  if (joint_mask != nullptr) {
+    a.key_mask = joint_mask;
+    a.mask_batch_stride = static_cast<long long>(p->mask_batch_stride);
+    a.tile_list = static_cast<int*>(c->tile_list.p);
+    a.tile_list_stride = static_cast<long long>(tile_list_ints(s));
+  }
   ZD_CUDA(c, zdraw::launch_qk_norm_rope(stream, a, p->in_dtype == ZDRAW_DTYPE_F32));
   return ZDRAW_CUDA_OK;
 }
 
-// q16/k16: fp16 in the given layout (token-major uses ld_q/ld_k). v in in_dtype, token-major.
-int run_attention(Ctx* c, cudaStream_t stream, const void* q16, const void* k16, bool qk_head_major,
-                  long long ld_q16, long long ld_k16, const void* v, const float* key_mask, void* o,
-                  const zdraw_cuda_attn_params* p, const Shape& s) {
+int check_attention(Ctx* c, const void* q16, const void* k16, const void* v, const float* key_mask, const void* o,
+                    const zdraw_cuda_attn_params* p) {
   if (!q16 || !k16 || !v || !o) return fail(c, ZDRAW_CUDA_E_ARG, "null tensor given to attention");
   if (!aligned16(q16) || !aligned16(k16) || !aligned16(v) || !aligned16(o))
     return fail(c, ZDRAW_CUDA_E_ARG, "tensor given to attention is not 16-byte aligned");
   if (p->has_key_mask && (!key_mask || !aligned16(key_mask)))
     return fail(c, ZDRAW_CUDA_E_ARG, "has_key_mask set but key_mask is null or misaligned");
+  return ZDRAW_CUDA_OK;
+}
+
+// q16/k16: fp16 in the given layout (token-major uses ld_q/ld_k). v in in_dtype, token-major.
+// prepared: the prologue launch before this one has cast v and written the tile lists (joint call).
+int run_attention(Ctx* c, cudaStream_t stream, const void* q16, const void* k16, bool qk_head_major,
+                  long long ld_q16, long long ld_k16, const void* v, const float* key_mask, void* o,
+                  const zdraw_cuda_attn_params* p, const Shape& s, bool prepared = false) {
+  int rc = check_attention(c, q16, k16, v, key_mask, o, p);
+  if (rc) return rc;
   const float* mask = p->has_key_mask ? key_mask : nullptr;
 
   // f32 v: cast into scratch (dense token-major), as the reference converts v before its
@@ -189,11 +210,12 @@ int run_attention(Ctx* c, cudaStream_t stream, const void* q16, const void* k16,
   const void* v16 = v;
   long long ld_v16 = s.ld_v;
   if (p->in_dtype == ZDRAW_DTYPE_F32) {
-    int rc = ensure(c, c->v16, qk16_bytes(s));
-    if (rc) return rc;
-    ZD_CUDA(c, zdraw::launch_cast_f32_to_f16(stream, static_cast<const float*>(v), c->v16.p,
-                                             static_cast<long long>(s.batch) * s.tokens, s.heads * kHeadDim,
-                                             s.ld_v));
+    if (!prepared) {
+      if ((rc = ensure(c, c->v16, qk16_bytes(s))) != 0) return rc;
+      ZD_CUDA(c, zdraw::launch_cast_f32_to_f16(stream, static_cast<const float*>(v), c->v16.p,
+                                               static_cast<long long>(s.batch) * s.tokens, s.heads * kHeadDim,
+                                               s.ld_v));
+    }
     v16 = c->v16.p;
     ld_v16 = static_cast<long long>(s.heads) * kHeadDim;
   }
@@ -239,7 +261,6 @@ int run_attention(Ctx* c, cudaStream_t stream, const void* q16, const void* k16,
   }
 
   CUtensorMap tm_q, tm_k, tm_v;
-  int rc;
   if ((rc = make_tmap(c, &tm_q, q16, qk_head_major, s, ld_q16)) != 0) return rc;
   if ((rc = make_tmap(c, &tm_k, k16, qk_head_major, s, ld_k16)) != 0) return rc;
   if ((rc = make_tmap(c, &tm_v, v16, false, s, ld_v16)) != 0) return rc;
@@ -260,9 +281,11 @@ int run_attention(Ctx* c, cudaStream_t stream, const void* q16, const void* k16,
   a.tile_list_stride = 0;
   if (mask) {
     const size_t ints = tile_list_ints(s);
-    if ((rc = ensure(c, c->tile_list, ints * s.batch * sizeof(int))) != 0) return rc;
-    ZD_CUDA(c, zdraw::launch_mask_prepare(stream, mask, a.mask_batch_stride, s.tokens, s.batch,
-                                          static_cast<int*>(c->tile_list.p), static_cast<long long>(ints)));
+    if (!prepared) {
+      if ((rc = ensure(c, c->tile_list, ints * s.batch * sizeof(int))) != 0) return rc;
+      ZD_CUDA(c, zdraw::launch_mask_prepare(stream, mask, a.mask_batch_stride, s.tokens, s.batch,
+                                            static_cast<int*>(c->tile_list.p), static_cast<long long>(ints)));
+    }
     a.tile_list = static_cast<const int*>(c->tile_list.p);
     a.tile_list_stride = static_cast<long long>(ints);
   }
@@ -301,10 +324,13 @@ int joint(Ctx* c, cudaStream_t stream, const void* q, const void* k, const void*
           const Shape& s) {
   int rc = reserve_scratch(c, p, s, true);
   if (rc) return rc;
-  rc = run_prologue(c, stream, q, k, q_w_txt, q_w_img, k_w_txt, k_w_img, rope_cos, rope_sin, c->q16.p, c->k16.p,
-                    true, p, s);
+  // What the attention part would refuse is refused before the prologue launch reads v and the mask.
+  rc = check_attention(c, c->q16.p, c->k16.p, v, key_mask, o, p);
   if (rc) return rc;
-  return run_attention(c, stream, c->q16.p, c->k16.p, true, 0, 0, v, key_mask, o, p, s);
+  rc = run_prologue(c, stream, q, k, q_w_txt, q_w_img, k_w_txt, k_w_img, rope_cos, rope_sin, c->q16.p, c->k16.p,
+                    true, p, s, v, p->has_key_mask ? key_mask : nullptr);
+  if (rc) return rc;
+  return run_attention(c, stream, c->q16.p, c->k16.p, true, 0, 0, v, key_mask, o, p, s, true);
 }
 
 }  // namespace

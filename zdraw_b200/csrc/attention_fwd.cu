@@ -46,6 +46,7 @@
 
 #include <type_traits>
 
+#include "mask_tiles.cuh"
 #include "ptx.cuh"
 
 namespace zdraw {
@@ -103,10 +104,6 @@ constexpr uint32_t kStMma = 1u << 1;
 constexpr uint32_t kStSoftmax = 1u << 2;
 constexpr uint32_t kStWaitProbe = 1u << 8;  // the self-test kernel below
 constexpr uint32_t kStGatherWait = 1u << 9;  // gather_fence_kernel's poll gave up
-
-// Tile-list entries: K/V tile index, plus a flag for tiles the key mask covers partly.
-constexpr int kTileMixedFlag = 0x40000000;
-constexpr int kTileIndexMask = 0x3FFFFFFF;
 
 __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag,
                                          uint32_t* status, uint32_t code) {
@@ -1297,34 +1294,12 @@ __global__ void __launch_bounds__(64, 1) wait_timeout_probe_kernel(uint32_t* sta
   __syncthreads();
 }
 
-// ---------------------------------------------------------------------------
-// Key-mask tile classification. One block per image, 128 threads = one tile's keys.
-// A tile is left out when every one of its keys is masked (-inf or beyond the
-// sequence), listed plain when all 128 keys exist and carry mask 0, else listed
-// with the mixed flag. Tiles stay in ascending order, so the reduction order over
-// keys does not depend on the mask.
-// ---------------------------------------------------------------------------
-__global__ void mask_prepare_kernel(const float* key_mask, long long mask_batch_stride, int tokens,
-                                    int n_kv_tiles, int* tile_list, long long list_stride) {
-  const float* mask = key_mask + static_cast<size_t>(blockIdx.x) * mask_batch_stride;
-  int* list = tile_list + static_cast<size_t>(blockIdx.x) * list_stride;
-  for (int j = 0; j < n_kv_tiles; ++j) {
-    const int key = j * kBN + static_cast<int>(threadIdx.x);
-    const bool exists = key < tokens;
-    const float mv = exists ? mask[key] : -INFINITY;
-    const int all_masked = __syncthreads_and(mv == -INFINITY);
-    const int all_zero = __syncthreads_and(exists && mv == 0.0f);
-    if (threadIdx.x == 0) list[1 + j] = all_masked ? -1 : (all_zero ? j : (j | kTileMixedFlag));
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int n = 0;
-    for (int j = 0; j < n_kv_tiles; ++j) {
-      const int e = list[1 + j];
-      if (e >= 0) list[1 + n++] = e;
-    }
-    list[0] = n;
-  }
+// Key-mask tile lists for the calls that have no prologue launch to carry them: one block per image.
+__global__ void __launch_bounds__(kMaskThreads) mask_prepare_kernel(const float* key_mask, long long mask_batch_stride,
+                                                                    int tokens, int n_kv_tiles, int* tile_list,
+                                                                    long long list_stride) {
+  classify_mask_tiles(key_mask + static_cast<size_t>(blockIdx.x) * mask_batch_stride, tokens, n_kv_tiles,
+                      tile_list + static_cast<size_t>(blockIdx.x) * list_stride);
 }
 
 }  // namespace
@@ -1450,7 +1425,7 @@ cudaError_t launch_attn_scalar(cudaStream_t stream, const ScalarArgs& args) {
 cudaError_t launch_mask_prepare(cudaStream_t stream, const float* key_mask, long long mask_batch_stride,
                                 int tokens, int batch, int* tile_list, long long list_stride) {
   const int n_kv_tiles = (tokens + kBN - 1) / kBN;
-  mask_prepare_kernel<<<batch, kBN, 0, stream>>>(key_mask, mask_batch_stride, tokens, n_kv_tiles, tile_list,
+  mask_prepare_kernel<<<batch, kMaskThreads, 0, stream>>>(key_mask, mask_batch_stride, tokens, n_kv_tiles, tile_list,
                                                  list_stride);
   return cudaGetLastError();
 }

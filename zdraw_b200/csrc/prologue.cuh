@@ -17,6 +17,16 @@ struct PrologueArgs {
   long long rope_batch_stride;                         // elements between images (0 = shared)
   void* q_out;  // f16
   void* k_out;
+  // Work of the joint call that the attention kernel needs as well and that runs as extra blocks of this
+  // launch: the cast of an f32 V (dense token-major f16; nullptr: none) and the tile lists of a key mask
+  // (nullptr: none), as launch_cast_f32_to_f16 and launch_mask_prepare make them.
+  const float* v = nullptr;
+  long long ld_v = 0;
+  void* v_out = nullptr;
+  const float* key_mask = nullptr;
+  long long mask_batch_stride = 0;
+  int* tile_list = nullptr;
+  long long tile_list_stride = 0;
 };
 
 cudaError_t launch_qk_norm_rope(cudaStream_t stream, const PrologueArgs& args, bool in_f32);
