@@ -410,18 +410,18 @@ ZDRAW_CUDA_API int zdraw_cuda_qkv_projection(void *ctx, void *stream, const void
  * giving half P; O = P V with f32 output), full, non-causal, no mask. q, k, v, o are DEVICE
  * pointers to [tokens][head_dim] f32. tokens (<= 65536) and head_dim (<= 4096) must be multiples
  * of 32, as the reference requires; else the call is declined. Scratch (half operands, tokens^2 half exp(scores),
- * e4m3 copies of Q and K for a first estimate of the row maxima, row statistics: 0.6 GB at 16384
+ * row statistics: 0.6 GB at 16384
  * tokens) is grow-only context memory; the f32 scores are never stored.
  */
 ZDRAW_CUDA_API int zdraw_cuda_wide_attention(void *ctx, void *stream, const float *q, const float *k, const float *v,
                                              float *o, size_t tokens, size_t head_dim);
 
 /*
- * Which way the last zdraw_cuda_wide_attention call on this context took its row maxima: 0 = from
- * the e4m3 copies of Q and K (admitted only when the operands' norms bound the error of every
- * estimated maximum below 2^6 in the exponentials), 1 = from the half operands (the reference's
- * exact form). The choice is made on the device from the data alone, so repeats take the same
- * route. Plays the part of the bridge's per-route counters (metal_api.m:350, 459). Synchronises
+ * Which way the last zdraw_cuda_wide_attention call on this context took its row maxima: 0 = from a
+ * sample of the keys, for every row (tried when the operands' norms keep the scores moderate; no row's
+ * maximum lay more than 2^16 above its sample in the exponentials), 1 = from all keys (the reference's
+ * exact form), for every row or for the blocks of 256 rows where the sample had missed it. The choice is
+ * made on the device from the data alone, so repeats take the same route. Plays the part of the bridge's per-route counters (metal_api.m:350, 459). Synchronises
  * `stream`.
  */
 ZDRAW_CUDA_API int zdraw_cuda_wide_attention_route(void *ctx, void *stream, uint32_t *exact_row_max);

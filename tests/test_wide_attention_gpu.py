@@ -142,3 +142,36 @@ def test_shapes_outside_the_kernels_are_declined(ctx):
     with pytest.raises(mattn.UnsupportedShape):
         ctx.wide_attention(x, x, x, o, mattn.Config(256, 1, 1, 512, causal=True))
     assert ctx.last_status() == 0
+
+
+@pytest.mark.parametrize("tokens", [1024, 1056, 2080, 4096])
+def test_keys_outside_the_sample_are_noticed(ctx, oracle, tokens):
+    """Row maxima come from every (tokens // 512)-th key; a key outside that sample that equals a query of usual norm
+    lies e^15 above the rest (512 / sqrt(512) = 22.6), beyond what the half range holds: that block of 256 rows (and
+    the last, ragged one) is done again from exact maxima, the others are not, and every row matches the oracle."""
+    dim = 512
+    q, k, v = make(tokens, dim, tokens)
+    hits = {301: 7, tokens - 1: tokens - 3}  # row -> key, no multiple of the stride (2, 2, 4, 8)
+    for r, j in hits.items():
+        k[j] = q[r]
+    cfg = mattn.Config(tokens, 1, 1, dim)
+    out = torch.full((tokens, dim), float("nan"), device="cuda")
+    ctx.wide_attention(q, k, v, out, cfg)
+    again = torch.full_like(out, float("nan"))
+    ctx.wide_attention(q, k, v, again, cfg)
+    in_place = q.clone()  # the result may take an operand's place
+    ctx.wide_attention(in_place, k, v, in_place, cfg)
+    torch.cuda.synchronize()
+    assert ctx.wide_attention_route() == 1 and ctx.last_status() == 0
+    assert torch.equal(out, again)
+    assert (out - in_place).abs().max() <= 1e-5  # f32 sums of the two halves of the keys, in one pass or two
+    got = out.cpu().numpy()
+    qh, kh, vh = q.cpu().numpy(), k.cpu().numpy(), v.cpu().numpy()
+    for r in (0, 255, 256, 301, 511, 512, tokens - 1):
+        want = oracle.sdpa(qh, kh, vh, heads=1, rows=(r, r + 1)).reshape(tokens, dim)[r]
+        err = np.abs(got[r] - want)
+        assert err.max() <= MAX_ABS and err.mean() <= MEAN_ABS, f"row {r}: {err.max()}"
+    assert np.allclose(got[301], vh[7], atol=4e-3)
+    q2, k2, v2 = make(tokens, dim, tokens + 1)
+    ctx.wide_attention(q2, k2, v2, out, cfg)
+    assert ctx.wide_attention_route() == 0  # the next call starts afresh

@@ -370,6 +370,7 @@ int zdraw_cuda_attn_create(int device, void** ctx_out) {
     delete c;
     return ZDRAW_CUDA_E_CUDA;
   }
+  c->wa_state = c->d_status + 32;  // zeroed with the status word
   *ctx_out = c;
   return ZDRAW_CUDA_OK;
 }
@@ -381,7 +382,7 @@ int zdraw_cuda_attn_destroy(void* ctx) {
   cudaDeviceSynchronize();
   Buf* bufs[] = {&c->q16, &c->k16, &c->v16, &c->tile_list, &c->st_q, &c->st_k, &c->st_v,
                  &c->st_o, &c->st_w, &c->st_cos, &c->st_sin, &c->st_mask,
-                 &c->wa_q16, &c->wa_k16, &c->wa_vt16, &c->wa_aux, &c->wa_p, &c->wa_q8, &c->wa_k8, &c->wa_stats};
+                 &c->wa_q16, &c->wa_k16, &c->wa_vt16, &c->wa_aux, &c->wa_p};
   for (Buf* b : bufs)
     if (b->p) cudaFree(b->p);
   if (c->d_status) cudaFree(c->d_status);

@@ -46,8 +46,8 @@ struct Ctx {
   Buf q16, k16, v16, tile_list;
   Buf st_q, st_k, st_v, st_o, st_w, st_cos, st_sin, st_mask;  // staging for the host-buffer path
   Buf wa_q16, wa_k16, wa_vt16, wa_aux, wa_p;  // wide-head attention: half operands, row statistics, exp(scores)
-  Buf wa_q8, wa_k8;                            // e4m3 copies of Q and K for the row-max pass
-  Buf wa_stats;                                // operand statistics (2 + 2 words) and the row-max route word
+  unsigned int* wa_state = nullptr;            // kWideStateWords words behind d_status (wide_attention.cuh)
+  bool wa_ran = false;                         // a wide attention call has been made
   // Device-resident RoPE tables for the host-buffer joint call (zdraw_cuda_attn_set_device_tables).
   const float* dev_cos = nullptr;
   const float* dev_sin = nullptr;

@@ -18,23 +18,27 @@ struct PartSpec {
   void* c;
   uint32_t epilogue;  // zdraw::kEpilogue*: 0 plain, 1 qk; 2 row max and 3 exp are internal (wide attention)
   const float *w_txt, *w_img;
-  const float* row_scale = nullptr;  // plain: optional factor per row
   unsigned int* row_key = nullptr;   // row max / exp: ordered keys of the row maxima
-  float* row_sum = nullptr;          // exp: partial row sums
-  const float* max_shift = nullptr;  // exp: optional amount subtracted from every row maximum
+  float* row_sum = nullptr;          // exp: partial row sums; plain: the rows are divided by their sum
+  int n_partial = 0;                 // partial sums per row
   float exp_scale = 0.0f;
   uint32_t n_valid = 0;              // row max / exp: real columns (0 = all n); W then has n_valid rows
 };
 
+// What only the wide attention's launches say.
+struct WideSpec {
+  uint32_t w_k_valid = 0;         // columns of W that exist when fewer than k (A has all k)
+  unsigned int* route = nullptr;  // device-side choice of the work (linear.cuh)
+  unsigned int* block_flags = nullptr;
+  int run_when = 0;
+  bool rows_first = false;        // tile order: across the column blocks of a row block first
+  int k_splits = 1;               // 2: C holds zeros and each tile's K is walked by two pairs (linear.cuh)
+};
+
 // Shared body of zdraw_cuda_linear and zdraw_cuda_qkv_projection: validates, builds the tensor
 // maps and launches one kernel that computes every part from the same A.
-// operands_e4m3 (internal, the row-max pass of the wide attention): A and W hold e4m3 bytes instead
-// of halves; p->a_dtype / w_dtype still say f16 and strides count elements.
 int run_linear(Ctx* cx, void* stream, const void* a, int n_parts, const PartSpec* parts, const float* rope_cos,
-               const float* rope_sin, const zdraw_cuda_linear_params* p, bool operands_e4m3 = false,
-               uint32_t w_k_valid = 0,  // columns of W that exist when fewer than k (A has all k)
-               const unsigned int* gate = nullptr, int gate_run_if = 0,  // device-side launch gate (linear.cuh)
-               bool rows_first = false) {  // tile order: across the column blocks of a row block first
+               const float* rope_sin, const zdraw_cuda_linear_params* p, const WideSpec& wide = WideSpec()) {
   if (!p) return fail(cx, ZDRAW_CUDA_E_ARG, "params is null");
   if (p->reserved != 0 || p->m == 0 || p->n == 0 || p->k == 0) return fail(cx, ZDRAW_CUDA_E_ARG, "zero size or reserved != 0");
   if (p->c_dtype != ZDRAW_DTYPE_F16 && p->c_dtype != ZDRAW_DTYPE_F32) return fail(cx, ZDRAW_CUDA_E_ARG, "bad c_dtype");
@@ -54,23 +58,23 @@ int run_linear(Ctx* cx, void* stream, const void* a, int n_parts, const PartSpec
   if (p->n % 32 != 0 || p->k % 32 != 0) return fail(cx, ZDRAW_CUDA_DECLINED, "n and k must be multiples of 32");
   if (p->m > (1u << 30) || p->n > (1u << 30) || p->k > (1u << 30)) return fail(cx, ZDRAW_CUDA_DECLINED, "shape too large");
   const long long ld_a = p->ld_a ? static_cast<long long>(p->ld_a) : p->k;
-  const long long ld_w = p->ld_w ? static_cast<long long>(p->ld_w) : (w_k_valid ? w_k_valid : p->k);
+  const long long ld_w = p->ld_w ? static_cast<long long>(p->ld_w) : (wide.w_k_valid ? wide.w_k_valid : p->k);
   const long long ld_c = p->ld_c ? static_cast<long long>(p->ld_c) : p->n;
-  if (ld_a < p->k || ld_w < static_cast<long long>(w_k_valid ? w_k_valid : p->k) || ld_c < p->n)
+  if (ld_a < p->k || ld_w < static_cast<long long>(wide.w_k_valid ? wide.w_k_valid : p->k) || ld_c < p->n)
     return fail(cx, ZDRAW_CUDA_E_ARG, "row stride smaller than the row");
-  const long long ld_align = operands_e4m3 ? 16 : 8;  // TMA strides are multiples of 16 bytes
-  if (ld_a % ld_align != 0 || ld_w % ld_align != 0 || ld_c % 8 != 0)
-    return fail(cx, ZDRAW_CUDA_DECLINED, "row strides must be multiples of 8 elements (16 for 8-bit operands)");
+  if (ld_a % 8 != 0 || ld_w % 8 != 0 || ld_c % 8 != 0)  // TMA strides are multiples of 16 bytes
+    return fail(cx, ZDRAW_CUDA_DECLINED, "row strides must be multiples of 8 elements");
   zdraw::LinearArgs la = {};
   la.m = static_cast<int>(p->m);
   la.n = static_cast<int>(p->n);
   la.k = static_cast<int>(p->k);
-  la.fp8 = operands_e4m3 ? 1 : 0;
   la.n_parts = n_parts;
   la.status = cx->d_status;
-  la.gate = gate;
-  la.gate_run_if = gate_run_if;
-  la.rows_first = rows_first ? 1 : 0;
+  la.route = wide.route;
+  la.block_flags = wide.block_flags;
+  la.run_when = wide.run_when;
+  la.rows_first = wide.rows_first ? 1 : 0;
+  la.k_splits = wide.k_splits;
   if (any_qk) {
     if (p->tokens == 0 || p->heads == 0 || p->m % p->tokens != 0 || p->n != p->heads * 128u || p->txt_tokens > p->tokens)
       return fail(cx, ZDRAW_CUDA_E_ARG, "qk epilogue needs m = images * tokens and n = heads * 128");
@@ -97,34 +101,37 @@ int run_linear(Ctx* cx, void* stream, const void* a, int n_parts, const PartSpec
     } else {
       lp.c_f32 = p->c_dtype == ZDRAW_DTYPE_F32;
       lp.ld_c = ld_c;
-      lp.row_scale = parts[i].row_scale;
       lp.row_key = parts[i].row_key;
       lp.row_sum = parts[i].row_sum;
-      lp.max_shift = parts[i].max_shift;
+      lp.n_partial = parts[i].n_partial;
       lp.exp_scale = parts[i].exp_scale;
       lp.n_valid = static_cast<int>(parts[i].n_valid ? parts[i].n_valid : p->n);
     }
   }
   ZD_CUDA(cx, cudaSetDevice(cx->device));
+  int pairs = 0;
+  ZD_CUDA(cx, zdraw::linear_pairs(cx->sm_count, &pairs));
   // Row-major matrices [rows][ld] as tiled tensor maps: boxes of 128 bytes (64 halves) x 128 rows.
   zdraw::LinearMaps maps;
   const cuuint32_t estr[4] = {1, 1, 1, 1};
-  const cuuint64_t esz = operands_e4m3 ? 1u : 2u;
   // Rows and columns beyond what a matrix has are filled with zeros by the copy engine.
   auto encode = [&](CUtensorMap* tm, const void* base_ptr, uint64_t rows, long long ld, uint64_t cols) {
     const cuuint64_t dims[4] = {cols, rows, 1, 1};
-    const cuuint64_t strides[3] = {esz * static_cast<cuuint64_t>(ld), esz * static_cast<cuuint64_t>(ld) * rows,
-                                   esz * static_cast<cuuint64_t>(ld) * rows};
-    const cuuint32_t box[4] = {operands_e4m3 ? 128u : 64u, 128, 1, 1};  // 128-byte rows either way
-    return cx->encode(tm, operands_e4m3 ? CU_TENSOR_MAP_DATA_TYPE_UINT8 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
-                      const_cast<void*>(base_ptr), dims, strides, box, estr,
+    const cuuint64_t strides[3] = {2u * static_cast<cuuint64_t>(ld), 2u * static_cast<cuuint64_t>(ld) * rows,
+                                   2u * static_cast<cuuint64_t>(ld) * rows};
+    const cuuint32_t box[4] = {64u, 128u, 1, 1};
+    return cx->encode(tm, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void*>(base_ptr), dims, strides, box, estr,
                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   };
-  if (encode(&maps.a, a, p->m, ld_a, p->k) != CUDA_SUCCESS) return fail(cx, ZDRAW_CUDA_E_CUDA, "cuTensorMapEncodeTiled failed");
+  if (encode(&maps.a, a, p->m, ld_a, p->k) != CUDA_SUCCESS)
+    return fail(cx, ZDRAW_CUDA_E_CUDA, "cuTensorMapEncodeTiled failed");
   for (int i = 0; i < zdraw::kMaxLinearParts; ++i) {
-    const PartSpec& ps = parts[i < n_parts ? i : 0];
-    if (encode(&maps.w[i], ps.w, ps.n_valid ? ps.n_valid : p->n, ld_w, w_k_valid ? w_k_valid : p->k) != CUDA_SUCCESS)
+    maps.w[i] = maps.w[0];  // unused entries
+    if (i >= n_parts) continue;
+    const PartSpec& ps = parts[i];
+    if (encode(&maps.w[i], ps.w, ps.n_valid ? ps.n_valid : p->n, ld_w, wide.w_k_valid ? wide.w_k_valid : p->k) !=
+        CUDA_SUCCESS)
       return fail(cx, ZDRAW_CUDA_E_CUDA, "cuTensorMapEncodeTiled failed");
   }
   // Plain parts: C for the epilogue's tile stores (32 columns x 32 rows, swizzle of the row size).
@@ -141,7 +148,7 @@ int run_linear(Ctx* cx, void* stream, const void* a, int n_parts, const PartSpec
                    CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
       return fail(cx, ZDRAW_CUDA_E_CUDA, "cuTensorMapEncodeTiled failed for C");
   }
-  ZD_CUDA(cx, zdraw::launch_linear(static_cast<cudaStream_t>(stream), maps, la, cx->sm_count));
+  ZD_CUDA(cx, zdraw::launch_linear(static_cast<cudaStream_t>(stream), maps, la, pairs));
   return ZDRAW_CUDA_OK;
 }
 
@@ -175,59 +182,91 @@ int zdraw_cuda_wide_attention(void* ctx, void* stream, const float* q, const flo
     return fail(cx, ZDRAW_CUDA_DECLINED, "tokens (<= 65536) and head_dim (<= 4096) must be multiples of 32");
   ZD_CUDA(cx, cudaSetDevice(cx->device));
   const size_t n = tokens * head_dim;
-  // The score matrix is tiled in blocks of 256 keys: its columns are padded to that (the padding
+  // The score matrix is tiled in blocks of up to 256 keys: its columns are padded to that (the padding
   // is stored as zeros and skipped by the row maximum).
   const size_t n_pad = (tokens + 255) / 256 * 256;
-  const size_t n_partial = 2 * (n_pad / 256);  // partial row sums: one per 128-column half tile
-  const size_t aux_bytes = tokens * 4 * (2 + n_partial);  // row keys, 1/row sum, partial sums
+  const size_t n_partial = n_pad / 128;  // partial row sums: one per 128 columns
+  const size_t n_blocks = (tokens + 255) / 256;
+  const size_t aux_bytes = 4 * (tokens * n_partial + tokens + n_blocks);  // partial sums, row keys, flags of 256 rows
   int rc;
   if ((rc = ensure(cx, cx->wa_q16, n * 2)) || (rc = ensure(cx, cx->wa_k16, n * 2)) || (rc = ensure(cx, cx->wa_vt16, n * 2)) ||
-      (rc = ensure(cx, cx->wa_aux, aux_bytes)) || (rc = ensure(cx, cx->wa_p, tokens * n_pad * 2)) ||
-      (rc = ensure(cx, cx->wa_q8, n)) || (rc = ensure(cx, cx->wa_k8, n)) || (rc = ensure(cx, cx->wa_stats, 256)))
+      (rc = ensure(cx, cx->wa_aux, aux_bytes)) || (rc = ensure(cx, cx->wa_p, tokens * n_pad * 2)))
     return rc;
-  unsigned int* stats = static_cast<unsigned int*>(cx->wa_stats.p);  // [0,1] Q, [2,3] K, [4] route, [5] shift of the estimated maxima
-  const float exp_scale = 1.4426950408889634f / std::sqrt(static_cast<float>(head_dim));
-  unsigned int* row_key = static_cast<unsigned int*>(cx->wa_aux.p);
-  float* row_inv = reinterpret_cast<float*>(row_key + tokens);
-  float* row_sum = row_inv + tokens;
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  // kf32_to_h x2, kvt_transpose_h (mvattn_owned.zig:322-330); Q and K also as e4m3 (see below)
-  ZD_CUDA(cx, cudaMemsetAsync(stats, 0, 32, st));
-  ZD_CUDA(cx, zdraw::launch_cast_f32_to_f16_e4m3(st, q, cx->wa_q16.p, cx->wa_q8.p, static_cast<long long>(tokens),
-                                                 static_cast<int>(head_dim), stats));
-  ZD_CUDA(cx, zdraw::launch_cast_f32_to_f16_e4m3(st, k, cx->wa_k16.p, cx->wa_k8.p, static_cast<long long>(tokens),
-                                                 static_cast<int>(head_dim), stats + 2));
-  ZD_CUDA(cx, zdraw::launch_wide_gate(st, stats, stats + 2, static_cast<int>(head_dim), exp_scale, stats + 4));
-  ZD_CUDA(cx, zdraw::launch_transpose_cast(st, v, cx->wa_vt16.p, static_cast<int>(tokens), static_cast<int>(head_dim)));
-  ZD_CUDA(cx, cudaMemsetAsync(row_key, 0, tokens * 4, st));  // key 0 lies below every float
-  // The scores S = Q K^T (K is already [n][k]) are never stored. A first product keeps only each
-  // row's maximum; a second one turns its accumulator into exp(scale (S - max)) in half and keeps
-  // partial row sums: recomputing S (k = head_dim is short) costs less than writing and re-reading
-  // tokens^2 f32 scores. Softmax does not change when another number than the exact maximum is
-  // subtracted, as long as nothing overflows, so the first product may run on e4m3 copies of Q and
-  // K at twice the rate - when the operands' norms prove its maxima close enough (wide_gate_kernel:
-  // within 2^6 of the true ones in the exponentials). Both forms of that product are enqueued and
-  // the route word picks the one that does the work; the other launch leaves at once. (The
-  // reference takes the exact f32 maximum of half products, krow_softmax_h,
-  // src/metal/mvattn_owned.zig:95-128; the half-operand route is that.)
+  float* row_sum = static_cast<float*>(cx->wa_aux.p);
+  unsigned int* row_key = reinterpret_cast<unsigned int*>(row_sum + tokens * n_partial);
+  unsigned int* block_flags = row_key + tokens;
+  zdraw::WideCast cast = {};
+  cast.q = q;
+  cast.k = k;
+  cast.v = v;
+  cast.q16 = cx->wa_q16.p;
+  cast.k16 = cx->wa_k16.p;
+  cast.vt16 = cx->wa_vt16.p;
+  cast.tokens = static_cast<int>(tokens);
+  cast.ch = static_cast<int>(head_dim);
+  cast.exp_scale = 1.4426950408889634f / std::sqrt(static_cast<float>(head_dim));
+  cast.row_key = row_key;
+  cast.block_flags = block_flags;
+  cast.state = cx->wa_state;
+  // O = P V has few tiles (tokens / 256 x head_dim / 256): where a second half-length round of work items
+  // fits the chip better, K is split and the halves are added to an O that the cast launch has zeroed.
+  int pairs = 0;
+  ZD_CUDA(cx, zdraw::linear_pairs(cx->sm_count, &pairs));
+  auto overlaps_o = [&](const float* x) { return x < o + n && o < x + n; };
+  const bool split = !overlaps_o(q) && !overlaps_o(k) && !overlaps_o(v) &&  // (an o in an operand's place is zeroed too early)
+                     zdraw::linear_split_pays(zdraw::linear_tiles(static_cast<int>(tokens), static_cast<int>(head_dim), 1), pairs);
+  cast.zero = split ? o : nullptr;
+  // kf32_to_h x2, kvt_transpose_h (mvattn_owned.zig:322-330)
+  ZD_CUDA(cx, zdraw::launch_wide_cast(static_cast<cudaStream_t>(stream), cast));
+  cx->wa_ran = true;
+  // The scores S = Q K^T (K is already [n][k]) are never stored. One product keeps only row maxima; a
+  // second one turns its accumulator into exp(scale (S - max)) in half and keeps partial row sums:
+  // recomputing S (k = head_dim is short) costs less than writing and re-reading tokens^2 f32 scores.
+  // Softmax does not change when another number than the maximum is subtracted, as long as nothing
+  // overflows, so the maxima come from some 512 keys spread over the image (every stride-th one, through
+  // the tensor map's row stride). A row whose largest score lies more than 2^16 above the sample's
+  // (in the exponentials) is noticed by the exp product; its block of 256 rows is then done again from the
+  // exact maxima by two launches that otherwise leave at once, as is everything when the operands' norms are
+  // too large for the sample to be worth trying (choose_route). All of it depends on the data alone. (The
+  // reference takes the exact f32 maximum of half products, krow_softmax_h, src/metal/mvattn_owned.zig:95-128.)
+  // Together with the split P V and the one cast launch: 94 -> 63 us at 4096 x 512, 759 -> 626 us at 16384 x 512,
+  // against row maxima from e4m3 copies of all keys. A call whose every block is done again takes about as much
+  // longer as one more exp product (26 and 275 us).
+  // Below 1024 tokens every key is in the sample: its maxima are exact and nothing can need doing again.
+  const size_t stride = tokens < 1024 ? 1 : tokens / 512;
+  const size_t n_sample = (tokens + stride - 1) / stride;
   zdraw_cuda_linear_params ps = {};
   ps.m = static_cast<uint32_t>(tokens);
-  ps.n = static_cast<uint32_t>(n_pad);
+  ps.n = static_cast<uint32_t>((n_sample + 255) / 256 * 256);
   ps.k = static_cast<uint32_t>(head_dim);
+  ps.ld_w = stride * head_dim;
+  ps.ld_c = n_pad;
   ps.a_dtype = ps.w_dtype = ps.c_dtype = ZDRAW_DTYPE_F16;
   PartSpec part_s = {cx->wa_k16.p, cx->wa_p.p, static_cast<uint32_t>(zdraw::kEpilogueRowMax), nullptr, nullptr};
   part_s.row_key = row_key;
-  part_s.n_valid = static_cast<uint32_t>(tokens);
-  part_s.w = cx->wa_k8.p;
-  if ((rc = run_linear(cx, stream, cx->wa_q8.p, 1, &part_s, nullptr, nullptr, &ps, true, 0, stats + 4, 0)) != 0) return rc;
-  part_s.w = cx->wa_k16.p;
-  if ((rc = run_linear(cx, stream, cx->wa_q16.p, 1, &part_s, nullptr, nullptr, &ps, false, 0, stats + 4, 1)) != 0) return rc;
-  part_s.epilogue = static_cast<uint32_t>(zdraw::kEpilogueExp);
   part_s.row_sum = row_sum;
-  part_s.exp_scale = exp_scale;
-  part_s.max_shift = reinterpret_cast<const float*>(stats + 5);
+  part_s.n_partial = static_cast<int>(n_partial);
+  part_s.exp_scale = cast.exp_scale;
+  part_s.n_valid = static_cast<uint32_t>(n_sample);
   if ((rc = run_linear(cx, stream, cx->wa_q16.p, 1, &part_s, nullptr, nullptr, &ps)) != 0) return rc;
-  ZD_CUDA(cx, zdraw::launch_row_sum_inverse(st, row_sum, static_cast<int>(n_partial), static_cast<long long>(tokens), row_inv));
+  ps.n = static_cast<uint32_t>(n_pad);
+  ps.ld_w = head_dim;
+  part_s.n_valid = static_cast<uint32_t>(tokens);
+  WideSpec when;
+  when.block_flags = block_flags;
+  if (stride > 1) {
+    when.route = cx->wa_state + zdraw::kWideRoute;
+    when.run_when = zdraw::kRunEstimate;
+  }
+  part_s.epilogue = static_cast<uint32_t>(zdraw::kEpilogueExp);
+  if ((rc = run_linear(cx, stream, cx->wa_q16.p, 1, &part_s, nullptr, nullptr, &ps, when)) != 0) return rc;
+  if (stride > 1) {
+    when.run_when = zdraw::kRunExact;
+    part_s.epilogue = static_cast<uint32_t>(zdraw::kEpilogueRowMax);
+    if ((rc = run_linear(cx, stream, cx->wa_q16.p, 1, &part_s, nullptr, nullptr, &ps, when)) != 0) return rc;
+    part_s.epilogue = static_cast<uint32_t>(zdraw::kEpilogueExp);
+    if ((rc = run_linear(cx, stream, cx->wa_q16.p, 1, &part_s, nullptr, nullptr, &ps, when)) != 0) return rc;
+  }
   // O[tokens, head_dim] = (P (V^T)^T) / row sum, f32 out
   zdraw_cuda_linear_params po = {};
   po.m = static_cast<uint32_t>(tokens);
@@ -237,20 +276,25 @@ int zdraw_cuda_wide_attention(void* ctx, void* stream, const float* q, const flo
   po.a_dtype = po.w_dtype = ZDRAW_DTYPE_F16;
   po.c_dtype = ZDRAW_DTYPE_F32;
   PartSpec part_o = {cx->wa_vt16.p, o, 0, nullptr, nullptr};
-  part_o.row_scale = row_inv;
-  return run_linear(cx, stream, cx->wa_p.p, 1, &part_o, nullptr, nullptr, &po, false, static_cast<uint32_t>(tokens),
-                    nullptr, 0, true);
+  part_o.row_sum = row_sum;
+  part_o.n_partial = static_cast<int>(n_partial);
+  WideSpec last;
+  last.w_k_valid = static_cast<uint32_t>(tokens);
+  last.rows_first = true;
+  last.k_splits = split ? 2 : 1;
+  return run_linear(cx, stream, cx->wa_p.p, 1, &part_o, nullptr, nullptr, &po, last);
 }
 
 int zdraw_cuda_wide_attention_route(void* ctx, void* stream, uint32_t* exact_row_max) {
   Ctx* cx = as_ctx(ctx);
   if (!cx || !exact_row_max) return ZDRAW_CUDA_E_ARG;
   *exact_row_max = 0;
-  if (!cx->wa_stats.p) return fail(cx, ZDRAW_CUDA_E_ARG, "no wide attention call has run on this context");
+  if (!cx->wa_ran) return fail(cx, ZDRAW_CUDA_E_ARG, "no wide attention call has run on this context");
   ZD_CUDA(cx, cudaSetDevice(cx->device));
   ZD_CUDA(cx, cudaStreamSynchronize(static_cast<cudaStream_t>(stream)));
-  ZD_CUDA(cx, cudaMemcpy(exact_row_max, static_cast<const unsigned int*>(cx->wa_stats.p) + 4, sizeof(uint32_t),
-                         cudaMemcpyDeviceToHost));
+  uint32_t route = 0;
+  ZD_CUDA(cx, cudaMemcpy(&route, cx->wa_state + zdraw::kWideRoute, sizeof(route), cudaMemcpyDeviceToHost));
+  *exact_row_max = route != 0 ? 1u : 0u;
   return ZDRAW_CUDA_OK;
 }
 

@@ -14,8 +14,7 @@
 //            the wide-head attention's softmax (the reference's krow_softmax_h,
 //            src/metal/mvattn_owned.zig:95-128), so its f32 scores never reach memory.
 //
-// Up to three products that share A run as one launch (the q, k and v projections), and A and W
-// may be e4m3 bytes (the row-max pass, tcgen05 kind::f8f6f4).
+// Up to three products that share A run as one launch (the q, k and v projections).
 //
 // Persistent, warp-specialised, one CTA pair (cluster of two, tcgen05 cta_group::2) per 256 x 256
 // tile of C: each CTA stages its own 128 rows of A and 128 of the tile's 256 rows of W
@@ -45,6 +44,9 @@ namespace {
 constexpr int kTM = 128;                 // rows of C per CTA (256 per pair)
 constexpr int kTN = 256;                 // columns of C per tile (two heads of 128)
 constexpr int kTK = 64;                  // K per stage: one 128-byte swizzled row of f16
+// Stages: 5 x 32 KB in flight per CTA. The launch of three projections at 1536 x 3072 x 3072 takes 71, 61
+// and 57 us with 3, 4 and 5: an L2 round trip with both barriers is what a stage hides.
+// (Tiles of 128 columns with up to 8 stages, for launches of few tiles, were no faster per tile than these.)
 constexpr int kStages = 5;
 constexpr int kABytes = kTM * kTK * 2;        // 16 KB: this CTA's rows of A
 constexpr int kBBytes = (kTN / 2) * kTK * 2;  // 16 KB: this CTA's half of the tile's rows of W
@@ -98,6 +100,13 @@ __device__ __forceinline__ uint32_t pack_clamped(float lo, float hi) {
 __global__ void __launch_bounds__(kThreads, 1)
 linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
+  if (a.route != nullptr) {
+    // A launch of the wide attention that may have nothing to do leaves before it sets anything up
+    // (both CTAs of a pair see the same word: it changes between 0 and 2 only while run_when is kRunEstimate).
+    grid_dependency_wait();
+    const unsigned int route = ld_volatile_u32(a.route);
+    if (a.run_when == kRunEstimate ? route == 1u : route == 0u) return;
+  }
   const uint32_t base = smem_u32(smem_raw);
   volatile uint32_t* flags = reinterpret_cast<volatile uint32_t*>(smem_raw + kOffFlags);
   volatile uint32_t* abort_flag = flags;
@@ -109,10 +118,13 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   const int tiles_n = (a.n + kTN - 1) / kTN;            // column blocks of one part (the last may be partial)
   const int tiles_m = (a.m + 2 * kTM - 1) / (2 * kTM);  // pair tiles: 256 rows
-  int n_tiles = tiles_m * tiles_n * a.n_parts;
+  // With k_splits == 2 a tile of C is computed twice, by neighbouring work items that each walk half of K
+  // and add their share to C.
+  const int n_items = tiles_m * tiles_n * a.n_parts * a.k_splits;
   // A stage is a 128-byte slice of K per row; rows, columns and K beyond the matrices read as zeros.
-  const int k_steps = a.fp8 ? (a.k + 2 * kTK - 1) / (2 * kTK) : (a.k + kTK - 1) / kTK;
-  const int k_per_stage = a.fp8 ? 2 * kTK : kTK;
+  const int k_steps_all = (a.k + kTK - 1) / kTK;
+  auto first_k = [&](int item) { return (item % a.k_splits) * (k_steps_all / a.k_splits); };
+  auto end_k = [&](int item) { return item % a.k_splits == a.k_splits - 1 ? k_steps_all : k_steps_all / a.k_splits; };
 
   if (threadIdx.x == 0) {
     // Both CTAs of a pair take every collective step below whatever happens, so a failed wait
@@ -147,8 +159,11 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
   tc_fence_after();
   const uint32_t tmem_base = flags[1];
   grid_dependency_wait();
-  // A gated launch that is not the chosen one has no tiles (both CTAs of a pair see the same word).
-  if (a.gate != nullptr && ((*a.gate != 0u) != (a.gate_run_if != 0))) n_tiles = 0;
+  grid_launch_dependents();  // the kernel behind this one may set itself up on SMs that run out of work
+  // When only some row blocks are to be done again, the others' tiles are passed over by every role alike.
+  const unsigned int* const block_flags =
+      (a.route != nullptr && a.run_when == kRunExact && ld_volatile_u32(a.route) == 2u) ? a.block_flags : nullptr;
+  auto passed_over = [&](int tile_m) -> bool { return block_flags != nullptr && ld_volatile_u32(block_flags + tile_m) == 0u; };
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -157,7 +172,8 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
       for (int pt = 0; pt < a.n_parts; ++pt) tma_prefetch_desc(&maps.w[pt]);
       uint32_t it = 0;
       bool ok = *abort_flag == 0u;
-      for (int tile = pair; tile < n_tiles && ok; tile += n_pairs) {
+      for (int item = pair; item < n_items && ok; item += n_pairs) {
+        const int tile = item / a.k_splits;
         // Consecutive tiles share the W block (part, tile_n) and walk down the rows: W stays in L2.
         // With rows_first they share the row block of A instead and walk across the column blocks:
         // the order for a long-K product whose A is the large operand (P V of the wide attention),
@@ -165,11 +181,12 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
         const int n_cols = tiles_n * a.n_parts;
         const int col = a.rows_first ? tile % n_cols : tile / tiles_m;
         const int tile_m = a.rows_first ? tile / n_cols : tile % tiles_m;
+        if (passed_over(tile_m)) continue;
         const int tile_n = col % tiles_n;
         const CUtensorMap* tm_w = &maps.w[col / tiles_n];
         const int row_a = (2 * tile_m + static_cast<int>(rank)) * kTM;
         const int row_w = tile_n * kTN + static_cast<int>(rank) * (kTN / 2);
-        for (int ks = 0; ks < k_steps; ++ks, ++it) {
+        for (int ks = first_k(item), ke = end_k(item); ks < ke; ++ks, ++it) {
           const uint32_t stage = it % kStages;
           const uint32_t phase = (it / kStages) & 1u;
           ok = wait_bar(bar(kBarEmpty + stage), phase ^ 1u, abort_flag, a.status);
@@ -178,8 +195,8 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
           // Both CTAs' bytes are counted on the even CTA's barrier, which expects all of them.
           const uint32_t full = cluster_map(bar(kBarFull + stage), 0);
           if (rank == 0) mbar_arrive_expect_tx(bar(kBarFull + stage), 2 * kStageBytes);
-          tma_load_4d_pair(dst, &maps.a, full, ks * k_per_stage, row_a, 0, 0);
-          tma_load_4d_pair(dst + kABytes, tm_w, full, ks * k_per_stage, row_w, 0, 0);
+          tma_load_4d_pair(dst, &maps.a, full, ks * kTK, row_a, 0, 0);
+          tma_load_4d_pair(dst + kABytes, tm_w, full, ks * kTK, row_w, 0, 0);
         }
       }
       if (!ok) {
@@ -194,7 +211,9 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
       uint32_t it = 0;
       int local = 0;
       bool ok = *abort_flag == 0u;
-      for (int tile = pair; tile < n_tiles && ok; tile += n_pairs, ++local) {
+      for (int item = pair; item < n_items && ok; item += n_pairs) {
+        const int tile = item / a.k_splits;
+        if (passed_over(a.rows_first ? tile / (tiles_n * a.n_parts) : tile % tiles_m)) continue;
         const int b = local & 1;
         const uint32_t use = static_cast<uint32_t>(local >> 1);
         // The epilogue warps must have drained this accumulator (first use passes at once).
@@ -202,35 +221,24 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
         if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + 256u * b;
-        // One K walk per operand type, so that the issuing thread's loop holds no type test.
-        auto walk_k = [&](auto is_fp8) {
-          for (int ks = 0; ks < k_steps; ++ks, ++it) {
-            const uint32_t stage = it % kStages;
-            const uint32_t phase = (it / kStages) & 1u;
-            ok = wait_bar(bar(kBarFull + stage), phase, abort_flag, a.status);
-            if (!ok) break;
-            const uint32_t a_addr = base + stage * kStageBytes;
-            const uint64_t desc_a = smem_desc_sw128(a_addr, 16, 1024);
-            const uint64_t desc_b = smem_desc_sw128(a_addr + kABytes, 16, 1024);
-            // Four MMAs per stage, each 32 bytes further along the swizzled rows: K = 16 halves
-            // or 32 e4m3 bytes.
+        const int k_first = first_k(item);
+        for (int ks = k_first, ke = end_k(item); ks < ke; ++ks, ++it) {
+          const uint32_t stage = it % kStages;
+          const uint32_t phase = (it / kStages) & 1u;
+          ok = wait_bar(bar(kBarFull + stage), phase, abort_flag, a.status);
+          if (!ok) break;
+          const uint32_t a_addr = base + stage * kStageBytes;
+          const uint64_t desc_a = smem_desc_sw128(a_addr, 16, 1024);
+          const uint64_t desc_b = smem_desc_sw128(a_addr + kABytes, 16, 1024);
+          // Four MMAs per stage, each 32 bytes (K = 16 halves) further along the swizzled rows.
 #pragma unroll
-            for (int kk = 0; kk < 4; ++kk) {
-              if constexpr (decltype(is_fp8)::value)
-                umma_ss_pair_f8(d_tmem, desc_a + 2u * kk, desc_b + 2u * kk, idesc, (ks > 0 || kk > 0) ? 1u : 0u);
-              else
-                umma_ss_pair(d_tmem, desc_a + 2u * kk, desc_b + 2u * kk, idesc, (ks > 0 || kk > 0) ? 1u : 0u);
-            }
-            umma_commit_pair(bar(kBarEmpty + stage), 3);  // both CTAs' producers may refill the stage
-          }
-        };
-        if (a.fp8) {
-          walk_k(std::true_type{});
-        } else {
-          walk_k(std::false_type{});
+          for (int kk = 0; kk < 4; ++kk)
+            umma_ss_pair(d_tmem, desc_a + 2u * kk, desc_b + 2u * kk, idesc, (ks > k_first || kk > 0) ? 1u : 0u);
+          umma_commit_pair(bar(kBarEmpty + stage), 3);  // both CTAs' producers may refill the stage
         }
         if (!ok) break;
         umma_commit_pair(bar(kBarAccFull + b), 3);  // both CTAs' epilogues may read their rows
+        ++local;
       }
       if (!ok) {
         umma_commit_pair(bar(kBarDrain), 1);
@@ -246,22 +254,41 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
     const int quarter = warp & 3;
     const int row = quarter * 32 + lane;
     const uint32_t lane_off = static_cast<uint32_t>(quarter * 32) << 16;
-    int local = 0;
+    int next_local = 0;
     bool ok = __all_sync(0xffffffffu, *abort_flag == 0u);  // warp-uniform
-    for (int tile = pair; tile < n_tiles && ok; tile += n_pairs, ++local) {
+    for (int item = pair; item < n_items && ok; item += n_pairs) {
+      const int tile = item / a.k_splits;
       const int n_cols = tiles_n * a.n_parts;
       const int col = a.rows_first ? tile % n_cols : tile / tiles_m;
-      const int tile_m = 2 * (a.rows_first ? tile / n_cols : tile % tiles_m) + static_cast<int>(rank);
+      const int pair_m = a.rows_first ? tile / n_cols : tile % tiles_m;  // block of 256 rows
+      if (passed_over(pair_m)) continue;
+      const int local = next_local++;
+      const int tile_m = 2 * pair_m + static_cast<int>(rank);
       const int tile_n = col % tiles_n;
+      const int half_n = 2 * tile_n + hh;  // this warpgroup's block of 128 columns
       const LinearPart& part = a.part[col / tiles_n];
       const int b = local & 1;
       const uint32_t use = static_cast<uint32_t>(local >> 1);
+      const long long m = static_cast<long long>(tile_m) * kTM + row;
+      const bool live = m < a.m;
+      float row_factor = 1.0f;  // plain with partial row sums: 1 / their sum, while the tile's MMAs run
+      if (part.epilogue == kEpiloguePlain && part.row_sum != nullptr && live) {
+        const float2* p2 = reinterpret_cast<const float2*>(part.row_sum + m * part.n_partial);
+        float s0 = 0.0f, s1 = 0.0f;
+#pragma unroll 8
+        for (int i = 0; i < part.n_partial / 2; ++i) {
+          const float2 v = p2[i];
+          s0 += v.x;
+          s1 += v.y;
+        }
+        const float sum = s0 + s1;
+        row_factor = sum > 0.0f ? 1.0f / sum : 0.0f;  // an empty row yields zeros, not NaN
+      }
       ok = __all_sync(0xffffffffu, wait_bar(bar(kBarAccFull + b), use & 1u, abort_flag, a.status));
       if (!ok) break;
       tc_fence_after();
-      const uint32_t t_acc = tmem_base + 256u * b + lane_off;
-      const long long m = static_cast<long long>(tile_m) * kTM + row;
-      const bool live = m < a.m;
+      // this warpgroup's 128 columns of the accumulator
+      const uint32_t t_acc = tmem_base + 256u * b + 128u * hh + lane_off;
       bool released = false;  // this warp has handed the accumulator back
 
       if (part.epilogue == kEpilogueRowMax) {
@@ -270,9 +297,9 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
 #pragma unroll 1
         for (int pc = 0; pc < 4; ++pc) {
           uint32_t x[32];
-          tmem_ld_x32(t_acc + 128u * hh + 32u * pc, x);
+          tmem_ld_x32(t_acc + 32u * pc, x);
           tmem_wait_ld();
-          const int col0 = tile_n * kTN + 128 * hh + 32 * pc;
+          const int col0 = 128 * half_n + 32 * pc;
           if (col0 + 32 <= part.n_valid) {
 #pragma unroll
             for (int i = 0; i < 32; i += 2) mx = max3(mx, __uint_as_float(x[i]), __uint_as_float(x[i + 1]));
@@ -294,23 +321,22 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
         uint4* stage = reinterpret_cast<uint4*>(smem_raw + kOffTab + (warp - 4) * kTabBytesPerWarp);
         const uint32_t stage_addr = base + kOffTab + (warp - 4) * kTabBytesPerWarp;
         const int row0 = tile_m * kTM + quarter * 32;  // first row of this warp
-        const int col_base = tile_n * kTN + 128 * hh;
+        const int col_base = 128 * half_n;
         const bool exp_mode = part.epilogue == kEpilogueExp;
-        // plain: optional factor of this row; exp: x -> exp2(x * c + bias), bias = -max * c
-        float mul = 1.0f, bias = 0.0f, psum = 0.0f;
+        // plain: factor of this row; exp: x -> exp2(x * c + bias), bias = -max * c
+        float mul = row_factor, bias = 0.0f;
+        uint64_t psum = 0ull;  // exp: sums of the even and of the odd columns (+0.0f, +0.0f)
         float top = -INFINITY;  // exp: largest raw score of the columns that exist
         if (exp_mode) {
           mul = part.exp_scale;
-          const float shift = part.max_shift ? *part.max_shift : 0.0f;
-          bias = live ? -(key_float(part.row_key[m]) - shift) * part.exp_scale : 0.0f;
-        } else if (part.row_scale != nullptr && live) {
-          mul = part.row_scale[m];
+          bias = live ? -key_float(part.row_key[m]) * part.exp_scale : 0.0f;
         }
+        const uint64_t mul2 = f2_pack(mul, mul), bias2 = f2_pack(bias, bias);
         if (part.c_f32) {
 #pragma unroll 1
           for (int pc = 0; pc < 4; ++pc) {  // 32 columns of this warp's 128 at a time
             uint32_t x[32];
-            tmem_ld_x32(t_acc + 128u * hh + 32u * pc, x);
+            tmem_ld_x32(t_acc + 32u * pc, x);
             tmem_wait_ld();
             // 128-byte rows, 128-byte swizzle, two 4 KB blocks
             const int buf = pc & 1;
@@ -325,7 +351,10 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
             fence_proxy_async_smem();  // this thread's writes, for the TMA engine
             __syncwarp();
             if (lane == 0 && row0 < a.m) {
-              tma_store_2d(tm_c, stage_addr + buf * 4096, col_base + 32 * pc, row0);
+              if (a.k_splits > 1)
+                tma_reduce_add_2d(tm_c, stage_addr + buf * 4096, col_base + 32 * pc, row0);
+              else
+                tma_store_2d(tm_c, stage_addr + buf * 4096, col_base + 32 * pc, row0);
               bulk_commit_group();
             }
           }
@@ -338,24 +367,26 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
           if (lane == 0) bulk_wait_group_read<0>();
           __syncwarp();
           uint32_t xa[32], xb[32];
-          tmem_ld_x32(t_acc + 128u * hh, xa);
+          tmem_ld_x32(t_acc, xa);
           auto piece = [&](int pc, const uint32_t* x) {
             uint4* st = stage + (pc >> 1) * 256;
             const int side = pc & 1;
             uint32_t h[16];
             if (exp_mode) {
-              // (the subtracted maximum may be an estimate, admitted only with a proven error bound:
-              // a score whose exponential would leave the half range means that bound was broken;
-              // the largest raw score is tracked for that check, one instruction per pair, and the
-              // conversion saturates at the largest finite half)
+              // (the subtracted maximum may be that of a sample of the keys: the largest raw score is
+              // tracked, one instruction per pair, and the conversion saturates at the largest finite
+              // half, so a row that the sample missed is noticed below and done again)
               const int n_live = part.n_valid - (col_base + 32 * pc);  // columns of this piece that exist
               if (n_live >= 32) {
 #pragma unroll
                 for (int i = 0; i < 16; ++i) {
-                  const float e0 = ex2_approx(fmaf(__uint_as_float(x[2 * i]), mul, bias));
-                  const float e1 = ex2_approx(fmaf(__uint_as_float(x[2 * i + 1]), mul, bias));
-                  top = max3(top, __uint_as_float(x[2 * i]), __uint_as_float(x[2 * i + 1]));
-                  psum += e0 + e1;  // f32 sum of the unrounded values, as the reference's softmax takes it
+                  const float x0 = __uint_as_float(x[2 * i]), x1 = __uint_as_float(x[2 * i + 1]);
+                  float e0, e1;
+                  f2_unpack(f2_fma(f2_pack(x0, x1), mul2, bias2), e0, e1);
+                  e0 = ex2_approx(e0);
+                  e1 = ex2_approx(e1);
+                  top = max3(top, x0, x1);
+                  psum = f2_add(psum, f2_pack(e0, e1));  // f32 sum of the unrounded values, as the reference's softmax takes it
                   h[i] = pack_f16x2_sat(e0, e1);
                 }
               } else {  // the ragged end of the row (at most once per row)
@@ -367,7 +398,7 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
                   if (2 * i + 1 >= n_live) e1 = 0.0f;
                   if (2 * i < n_live) top = fmaxf(top, __uint_as_float(x[2 * i]));
                   if (2 * i + 1 < n_live) top = fmaxf(top, __uint_as_float(x[2 * i + 1]));
-                  psum += e0 + e1;
+                  psum = f2_add(psum, f2_pack(e0, e1));
                   h[i] = pack_f16x2_sat(e0, e1);
                 }
               }
@@ -381,13 +412,13 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
               st[lane * 8 + ((4 * side + i) ^ (lane & 7))] = make_uint4(h[4 * i], h[4 * i + 1], h[4 * i + 2], h[4 * i + 3]);
           };
           tmem_wait_ld();
-          tmem_ld_x32(t_acc + 128u * hh + 32u, xb);
+          tmem_ld_x32(t_acc + 32u, xb);
           piece(0, xa);
           tmem_wait_ld();
-          tmem_ld_x32(t_acc + 128u * hh + 64u, xa);
+          tmem_ld_x32(t_acc + 64u, xa);
           piece(1, xb);
           tmem_wait_ld();
-          tmem_ld_x32(t_acc + 128u * hh + 96u, xb);
+          tmem_ld_x32(t_acc + 96u, xb);
           piece(2, xa);
           tmem_wait_ld();
           // The accumulator is in registers: the MMAs of the tile after next may have it now.
@@ -404,9 +435,20 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
             bulk_commit_group();
           }
         }
-        if (exp_mode && live) part.row_sum[m * (2 * tiles_n) + 2 * tile_n + hh] = psum;
-        // exp2 argument of the largest score: 16 is where the half range ends (NaN also reports).
-        if (exp_mode && live && top > -INFINITY && !(fmaf(top, mul, bias) < 15.99f)) atomicOr(a.status, kStExpClamp);
+        if (exp_mode && live) {
+          float even, odd;
+          f2_unpack(psum, even, odd);
+          part.row_sum[m * part.n_partial + half_n] = even + odd;
+          // exp2 argument of the largest score: 16 is where the half range ends (NaN also reports).
+          if (top > -INFINITY && !(fmaf(top, mul, bias) < 15.99f)) {
+            if (a.run_when == kRunEstimate) {  // a key outside the sample lies more than 2^16 above it
+              a.block_flags[pair_m] = 1u;
+              *a.route = 2u;
+            } else {
+              atomicOr(a.status, kStExpClamp);
+            }
+          }
+        }
       } else {
         // qk epilogue: the tile's 256 columns are two heads of this token's projection.
         // Its cos/sin rows are parked in the per-warp block that a plain or exp epilogue of an
@@ -424,9 +466,9 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
 #pragma unroll
         for (int it = 0; it < 4; ++it) roff[it] = __shfl_sync(0xffffffffu, my_off, it * 8 + (lane >> 2)) + 4 * (lane & 3);
         float4* tab = reinterpret_cast<float4*>(smem_raw + kOffTab + (warp - 4) * kTabBytesPerWarp);
-        if (tile_n * 2 + hh < a.heads) {  // an odd head count leaves the last tile's second half empty
-          const int head = tile_n * 2 + hh;
-          const uint32_t t_head = t_acc + 128u * hh;
+        if (half_n < a.heads) {  // an odd head count leaves the second half of the last 256-column tile empty
+          const int head = half_n;
+          const uint32_t t_head = t_acc;
           // pass 1: sum of squares over the head's 128 columns (f32, as the reference's GPU kernels)
           float ss0 = 0.f, ss1 = 0.f, ss2 = 0.f, ss3 = 0.f;
 #pragma unroll 1
@@ -525,21 +567,26 @@ cudaError_t linear_configure() {
   return cudaFuncSetAttribute(linear_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
 }
 
-cudaError_t launch_linear(cudaStream_t stream, const LinearMaps& maps, const LinearArgs& args, int sm_count) {
-  const int n_tiles = ((args.m + 2 * kTM - 1) / (2 * kTM)) * ((args.n + kTN - 1) / kTN) * args.n_parts;
-  cudaLaunchConfig_t cfg = {};
-  cfg.blockDim = dim3(kThreads);
-  cfg.dynamicSmemBytes = kSmemBytes;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[2];
+namespace {
+
+void launch_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, cudaStream_t stream) {
+  *cfg = {};
+  cfg->blockDim = dim3(kThreads);
+  cfg->dynamicSmemBytes = kSmemBytes;
+  cfg->stream = stream;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = 2;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 2;
+  cfg->attrs = attr;
+  cfg->numAttrs = 2;
+}
+
+}  // namespace
+
+cudaError_t linear_pairs(int sm_count, int* out) {
   // One resident CTA pair per two SMs; how many pairs the device can hold at once is asked once
   // per device (a pair needs two SMs of one GPC).
   static int pairs_of_device[64] = {};
@@ -548,6 +595,9 @@ cudaError_t launch_linear(cudaStream_t stream, const LinearMaps& maps, const Lin
   if (err != cudaSuccess) return err;
   int pairs = (device >= 0 && device < 64) ? pairs_of_device[device] : 0;
   if (pairs == 0) {
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr[2];
+    launch_config(&cfg, attr, nullptr);
     cfg.gridDim = dim3(2 * (sm_count / 2));
     err = cudaOccupancyMaxActiveClusters(&pairs, linear_kernel, &cfg);
     if (err != cudaSuccess) return err;
@@ -555,6 +605,15 @@ cudaError_t launch_linear(cudaStream_t stream, const LinearMaps& maps, const Lin
     if (pairs > sm_count / 2) pairs = sm_count / 2;
     if (device >= 0 && device < 64) pairs_of_device[device] = pairs;
   }
+  *out = pairs;
+  return cudaSuccess;
+}
+
+cudaError_t launch_linear(cudaStream_t stream, const LinearMaps& maps, const LinearArgs& args, int pairs) {
+  const int n_tiles = linear_tiles(args.m, args.n, args.n_parts) * args.k_splits;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr[2];
+  launch_config(&cfg, attr, stream);
   cfg.gridDim = dim3(2 * (n_tiles < pairs ? n_tiles : pairs));
   return cudaLaunchKernelEx(&cfg, linear_kernel, maps, args);
 }

@@ -12,6 +12,8 @@ constexpr int kEpilogueQk = 1;      // q/k prologue applied to the accumulator
 constexpr int kEpilogueRowMax = 2;  // no C: row_key[row] = max over the row, as an ordered key
 constexpr int kEpilogueExp = 3;     // C = half(exp2((A W^T - max[row]) * exp_scale)), partial row sums
 
+constexpr int kRunEstimate = 1, kRunExact = 2;  // LinearArgs::run_when
+
 constexpr int kMaxLinearParts = 3;
 
 // One output of a launch: C_p[m, n] = A[m, k] * W_p[n, k]^T with its own epilogue.
@@ -21,14 +23,14 @@ struct LinearPart {
   void* c;       // plain: [m][ld_c]; qk: f16 head-major [image][head][token][128]
   long long ld_c;
   const float *w_txt, *w_img;  // qk: norm weights [128]
-  // plain: optional per-row factor [m]. row max: out, one ordered key per row (see float_key), zeroed
-  // by the caller. exp: in, the same keys; row_sum receives [m][2 * n / 256] partial sums of the
-  // exponentials (f32, before rounding to half), one per 128-column half tile.
-  const float* row_scale;
+  // row max: out, one ordered key per row (see float_key), zeroed by the caller. exp: in, the same keys;
+  // row_sum receives [m][n_partial] partial sums of the exponentials (f32, before rounding to half), one
+  // per 128 columns. plain: with row_sum the rows are divided by the sum of their partial sums (added in
+  // a fixed order). n_partial is even.
   unsigned int* row_key;
   float* row_sum;
+  int n_partial;
   float exp_scale;
-  const float* max_shift;  // exp: optional, one float: subtracted from every row maximum before use
   // row max / exp: columns at and beyond n_valid are padding of the last column block (W has no
   // such rows): they do not count for the maximum and are stored as zeros.
   int n_valid;
@@ -36,11 +38,13 @@ struct LinearPart {
 
 // Up to three products that share A (the Q, K and V projections of one activation) run as one
 // launch over n_parts * (n / 256) column blocks. A and every W are reached through tensor maps
-// (f16, 128-byte swizzle, boxes of 64 columns x 128 rows; e4m3: boxes of 128 columns). Tiles are
-// 256 columns x 64 (e4m3: 128) of K; partial tiles read zeros beyond the matrices.
+// (f16, 128-byte swizzle, boxes of 64 columns x 128 rows). Tiles are
+// 256 columns x 64 of K; partial tiles read zeros beyond the matrices.
 struct LinearArgs {
   int m, n, k;
-  int fp8;  // 1: A and W are e4m3 bytes (k % 128 == 0), a 128-byte swizzled row holds 128 elements
+  // 1, or 2 (f32 plain C that holds zeros before the launch, k > 64): each tile's K is walked in two halves by
+  // two CTA pairs that add their results to C. Two additions to zero give the same sum in either order.
+  int k_splits;
   int n_parts;
   LinearPart part[kMaxLinearParts];
   // qk epilogue (n == heads * 128, m == images * tokens)
@@ -49,11 +53,14 @@ struct LinearArgs {
   const float *rope_cos, *rope_sin;  // [tokens][128]
   long long rope_batch_stride;
   uint32_t* status;
-  // Optional launch gate: when set, the kernel does its work only if (*gate != 0) == (gate_run_if != 0),
-  // read after the preceding kernel in the stream has finished; otherwise every CTA leaves at once.
-  // Lets the host enqueue two alternative launches and a device-side decision pick one.
-  const unsigned int* gate;
-  int gate_run_if;
+  // Launches of the wide attention that a word in device memory decides on (nullptr: always runs).
+  // *route is 0 (row maxima come from a sample of the keys), 1 (exact maxima for every row) or 2 (exact
+  // maxima for the blocks of 256 rows whose flag is set: a score left the half range). A kRunEstimate launch
+  // leaves at once when it is 1, and its exp epilogue sets the flags and the 2; a kRunExact launch
+  // leaves at once when it is 0 and passes over the blocks that are not flagged when it is 2.
+  unsigned int* route;
+  unsigned int* block_flags;
+  int run_when;
   // Tile order: 0 = down the rows of one column block (W stays in L2), 1 = across the column blocks
   // of one row block (A stays in L2).
   int rows_first;
@@ -69,6 +76,15 @@ struct LinearMaps {
 };
 
 cudaError_t linear_configure();
-cudaError_t launch_linear(cudaStream_t stream, const LinearMaps& maps, const LinearArgs& args, int sm_count);
+// CTA pairs that the current device holds at once.
+cudaError_t linear_pairs(int sm_count, int* pairs);
+// Tiles of 256 x 256 of a launch, and whether splitting their K in two lets it end sooner: each pair takes whole
+// work items, so a launch lasts as long as its busiest pair's items. (4096 x 512 x 4096: 32 tiles on 74 pairs,
+// 64 half-length items when split.)
+inline int linear_tiles(int m, int n, int n_parts) { return ((m + 255) / 256) * ((n + 255) / 256) * n_parts; }
+inline bool linear_split_pays(int tiles, int pairs) {
+  return (2 * tiles + pairs - 1) / pairs < 2 * ((tiles + pairs - 1) / pairs);
+}
+cudaError_t launch_linear(cudaStream_t stream, const LinearMaps& maps, const LinearArgs& args, int pairs);
 
 }  // namespace zdraw

@@ -1,67 +1,69 @@
-// Helper kernels of the wide-head attention (one head, head_dim 512: the VAE mid-block shape), which
+// First kernel of the wide-head attention (one head, head_dim 512: the VAE mid-block shape), which
 // follows the reference's decomposition into GEMMs (src/metal/mvattn_owned.zig:283-330, product tier:
 // half Q, K and V^T, S = Q K^T with f32 output, a row softmax writing half P, O = P (V^T)^T), with
 // the softmax (krow_softmax_h, :95-128) folded into the epilogues of linear_kernel so that the f32
-// scores never reach memory. This file holds the transpose-and-cast of V (kvt_transpose_h, :84-94)
-// and the reduction of the partial row sums.
+// scores never reach memory. This file holds the casts of Q and K (kf32_to_h), the transpose-and-cast
+// of V (kvt_transpose_h, :84-94) and the choice of how the row maxima are taken.
 #include "wide_attention.cuh"
 
 #include <cuda_fp16.h>
-#include <cuda_fp8.h>
+
+#include "ptx.cuh"
 
 namespace zdraw {
 
 namespace {
 
 constexpr float kHalfMax = 65504.0f;
+constexpr int kRowsPerBlock = 8;  // Q, K: one warp per row
+constexpr int kVTile = 64;        // V: 64 tokens x 64 channels per block
 
-// 32 x 32 tiles through shared memory: coalesced 128-byte reads along ch, coalesced 64-byte
-// writes along tokens.
-__global__ void __launch_bounds__(256) transpose_cast_kernel(const float* __restrict__ in, __half* __restrict__ out,
-                                                             int tokens, int ch) {
-  __shared__ float tile[32][33];
-  const int t0 = blockIdx.x * 32, c0 = blockIdx.y * 32;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
+__device__ __forceinline__ float clamp_half(float x) { return fminf(fmaxf(x, -kHalfMax), kHalfMax); }
+
+// V: float4 reads along the channels, 128-byte writes along the tokens (two halves per lane).
+__device__ __forceinline__ void transpose_block(const WideCast& a, int block, __half (*tile)[kVTile + 2]) {
+  const int blocks_t = (a.tokens + kVTile - 1) / kVTile;
+  const int t0 = (block % blocks_t) * kVTile, c0 = (block / blocks_t) * kVTile;
+  const int piece = static_cast<int>(threadIdx.x) & 15, row = static_cast<int>(threadIdx.x) >> 4;
 #pragma unroll
-  for (int r = ty; r < 32; r += 8) {
-    const int t = t0 + r, c = c0 + tx;
-    tile[r][tx] = (t < tokens && c < ch) ? in[static_cast<long long>(t) * ch + c] : 0.0f;
+  for (int r = 0; r < kVTile; r += 16) {
+    const int t = t0 + r + row, c = c0 + 4 * piece;
+    float4 v = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (t < a.tokens && c < a.ch) v = __ldg(reinterpret_cast<const float4*>(a.v + static_cast<long long>(t) * a.ch + c));
+    tile[4 * piece + 0][r + row] = __float2half_rn(clamp_half(v.x));
+    tile[4 * piece + 1][r + row] = __float2half_rn(clamp_half(v.y));
+    tile[4 * piece + 2][r + row] = __float2half_rn(clamp_half(v.z));
+    tile[4 * piece + 3][r + row] = __float2half_rn(clamp_half(v.w));
   }
   __syncthreads();
+  const int lane = static_cast<int>(threadIdx.x) & 31, warp = static_cast<int>(threadIdx.x) >> 5;
+  __half* out = static_cast<__half*>(a.vt16);
 #pragma unroll
-  for (int r = ty; r < 32; r += 8) {
-    const int c = c0 + r, t = t0 + tx;
-    if (c < ch && t < tokens) {
-      const float v = fminf(fmaxf(tile[tx][r], -kHalfMax), kHalfMax);
-      out[static_cast<long long>(c) * tokens + t] = __float2half_rn(v);
-    }
+  for (int i = 0; i < kVTile / 8; ++i) {
+    const int c = 8 * i + warp, t = t0 + 2 * lane;
+    if (c0 + c < a.ch && t < a.tokens)
+      *reinterpret_cast<__half2*>(out + static_cast<long long>(c0 + c) * a.tokens + t) =
+          *reinterpret_cast<const __half2*>(&tile[c][2 * lane]);
   }
 }
 
-// One warp per row of [rows][ch] f32: four floats per lane and step -> four halves (clamped) and
-// four e4m3 bytes (saturating), so the operand is read once for both copies. The warp also takes
-// the row's sum of squares (each lane adds its elements in order, the lanes are folded by xor
-// shuffles: the same order on every run) and its largest magnitude; stats[0] / stats[1] receive the
-// maxima over all rows as float bits (non-negative floats order like unsigned integers, and a
-// maximum does not depend on the order of the updates): one update per block of eight rows, after
-// the block's warps have met in shared memory (two words that thousands of warps hit directly
-// cost more than the cast itself). NaN inputs set stats[1] to the NaN pattern.
-__global__ void __launch_bounds__(256) cast_f32_to_f16_e4m3_kernel(const float* __restrict__ in, __half* __restrict__ out16,
-                                                                   uint8_t* __restrict__ out8, long long rows, int ch,
-                                                                   unsigned int* __restrict__ stats) {
-  __shared__ unsigned int block_stats[2];
-  if (threadIdx.x < 2) block_stats[threadIdx.x] = 0u;
-  __syncthreads();
-  const long long row_raw = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
-  const bool live = row_raw < rows;
-  const long long row = live ? row_raw : rows - 1;  // a repeated row changes no maximum and is not stored
-  const int lane = threadIdx.x & 31;
-  const float4* src = reinterpret_cast<const float4*>(in + row * ch);
-  uint2* dst16 = reinterpret_cast<uint2*>(out16 + row * ch);
-  uint32_t* dst8 = reinterpret_cast<uint32_t*>(out8 + row * ch);
+// Q or K: one warp per row, four floats per lane and step -> four halves (clamped). The warp also takes
+// the row's sum of squares (each lane adds its elements in order, the lanes are folded by xor shuffles:
+// the same order on every run) and its largest magnitude; the block's maxima end in block_stats as float
+// bits (non-negative floats order like unsigned integers, and a maximum does not depend on the order of
+// the updates). NaN inputs set block_stats[1] to the NaN pattern.
+__device__ __forceinline__ void cast_block(const WideCast& a, const float* in, __half* out16, int block,
+                                           unsigned int* block_stats, bool zero_rows) {
+  const int row_raw = block * kRowsPerBlock + (static_cast<int>(threadIdx.x) >> 5);
+  const bool live = row_raw < a.tokens;
+  const long long row = live ? row_raw : a.tokens - 1;  // a repeated row changes no maximum and is not stored
+  const int lane = static_cast<int>(threadIdx.x) & 31;
+  const float4* src = reinterpret_cast<const float4*>(in + row * a.ch);
+  uint2* dst16 = reinterpret_cast<uint2*>(out16 + row * a.ch);
+  float4* zero = zero_rows ? reinterpret_cast<float4*>(a.zero + row * a.ch) : nullptr;
   float ss = 0.0f, amax = 0.0f;
   bool bad = false;
-  const int n4 = ch / 4;
+  const int n4 = a.ch / 4;
   // Four loads in flight per lane (512 floats per pass of the warp): the row of the VAE shape in one pass.
   for (int i0 = lane; i0 < n4; i0 += 128) {
     float4 vv[4];
@@ -70,27 +72,22 @@ __global__ void __launch_bounds__(256) cast_f32_to_f16_e4m3_kernel(const float* 
       if (i0 + 32 * u < n4) vv[u] = __ldg(src + i0 + 32 * u);
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
-    const int i = i0 + 32 * u;
-    if (i >= n4) break;
-    float4 v = vv[u];
-    ss = fmaf(v.x, v.x, ss);
-    ss = fmaf(v.y, v.y, ss);
-    ss = fmaf(v.z, v.z, ss);
-    ss = fmaf(v.w, v.w, ss);
-    amax = fmaxf(fmaxf(amax, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
-    bad = bad || !(v.x == v.x) || !(v.y == v.y) || !(v.z == v.z) || !(v.w == v.w);
-    v.x = fminf(fmaxf(v.x, -kHalfMax), kHalfMax);
-    v.y = fminf(fmaxf(v.y, -kHalfMax), kHalfMax);
-    v.z = fminf(fmaxf(v.z, -kHalfMax), kHalfMax);
-    v.w = fminf(fmaxf(v.w, -kHalfMax), kHalfMax);
-    const __half2 h0 = __floats2half2_rn(v.x, v.y), h1 = __floats2half2_rn(v.z, v.w);
-    uint2 o;
-    o.x = *reinterpret_cast<const uint32_t*>(&h0);
-    o.y = *reinterpret_cast<const uint32_t*>(&h1);
-    if (live) dst16[i] = o;
-    const uint32_t lo = __nv_cvt_float2_to_fp8x2(make_float2(v.x, v.y), __NV_SATFINITE, __NV_E4M3);
-    const uint32_t hi = __nv_cvt_float2_to_fp8x2(make_float2(v.z, v.w), __NV_SATFINITE, __NV_E4M3);
-    if (live) dst8[i] = lo | (hi << 16);
+      const int i = i0 + 32 * u;
+      if (i >= n4) break;
+      const float4 v = vv[u];
+      ss = fmaf(v.x, v.x, ss);
+      ss = fmaf(v.y, v.y, ss);
+      ss = fmaf(v.z, v.z, ss);
+      ss = fmaf(v.w, v.w, ss);
+      amax = fmaxf(fmaxf(amax, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
+      bad = bad || !(v.x == v.x) || !(v.y == v.y) || !(v.z == v.z) || !(v.w == v.w);
+      const __half2 h0 = __floats2half2_rn(clamp_half(v.x), clamp_half(v.y));
+      const __half2 h1 = __floats2half2_rn(clamp_half(v.z), clamp_half(v.w));
+      uint2 o;
+      o.x = *reinterpret_cast<const uint32_t*>(&h0);
+      o.y = *reinterpret_cast<const uint32_t*>(&h1);
+      if (live) dst16[i] = o;
+      if (zero && live) zero[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
   }
 #pragma unroll
@@ -103,75 +100,80 @@ __global__ void __launch_bounds__(256) cast_f32_to_f16_e4m3_kernel(const float* 
     atomicMax(block_stats + 0, __float_as_uint(ss));  // +inf orders above every finite value
     atomicMax(block_stats + 1, bad ? 0x7fc00000u : __float_as_uint(amax));
   }
+}
+
+// Whether the row maxima may come from a sample of the keys, from the operands' statistics alone. A
+// sampled maximum is never above the true one, so the largest exponential of a row is at least 1, and it
+// fits half as long as the true maximum lies less than 2^16 above the sampled one in the exponentials.
+// The exp product notices a row where it does not, and its block of 256 rows is done again from the exact maxima:
+// that costs a block as much as the exact route from the beginning plus the lost product, so the sample is only
+// tried while scores are moderate: largest norms |q| |k| * scale (which bounds every score) up to 81 in
+// units of the exponent, no value beyond 448, no NaN. (N(0,1) operands at 512 channels: 42.)
+__device__ __forceinline__ unsigned int choose_route(const unsigned int* stats, int ch, float exp_scale) {
+  const float nq = sqrtf(__uint_as_float(stats[kWideStatQ])), nk = sqrtf(__uint_as_float(stats[kWideStatK]));
+  const float aq = __uint_as_float(stats[kWideStatQ + 1]), ak = __uint_as_float(stats[kWideStatK + 1]);
+  const float e = 0.0625f, d = 0.0009765625f, n = static_cast<float>(ch);
+  const float spread = (2.0f * e + e * e) * nq * nk + d * (nq + nk) * sqrtf(n) + n * d * d;
+  return (aq <= 448.0f && ak <= 448.0f && spread * exp_scale <= 10.5f) ? 0u : 1u;  // 1 for NaN
+}
+
+// One launch for the three operands (three launches, two memsets and a one-thread kernel for the route took
+// about 25 us of a call at 4096 x 512, this takes 8). Memory-bound: 6 bytes per element, 26 us at 16384 x 512.
+__global__ void __launch_bounds__(256) wide_cast_kernel(const WideCast a, int row_blocks) {
+  __shared__ __half tile[kVTile][kVTile + 2];
+  __shared__ unsigned int block_stats[2];
+  // The launches before this one may still read what it writes.
+  grid_dependency_wait();
+  grid_launch_dependents();
+  const int block = static_cast<int>(blockIdx.x);
+  if (block >= 2 * row_blocks) {
+    transpose_block(a, block - 2 * row_blocks, tile);
+    return;
+  }
+  const bool is_k = block >= row_blocks;
+  if (threadIdx.x < 2) block_stats[threadIdx.x] = 0u;
   __syncthreads();
-  if (threadIdx.x < 2) atomicMax(stats + threadIdx.x, block_stats[threadIdx.x]);
-}
-
-// Decides, from the operands' statistics alone, whether row maxima taken from the e4m3 copies of Q
-// and K are close enough to the true ones. An e4m3 value differs from the half it was rounded from
-// by a factor within 1 +- 2^-4 (3 mantissa bits) or, below the smallest normal 2^-6, by at most
-// 2^-10; so for every score |q8 . k8 - q . k| <= (2 e + e^2) |q| |k| + d (|q| + |k|) sqrt(n) + n d^2
-// with e = 2^-4, d = 2^-10, n = head_dim (Cauchy-Schwarz). Let E be that bound in the units of the
-// exp2 argument. The half exponentials tolerate a subtracted maximum that is up to 15 too small
-// (the largest is then 2^15) but only about 6 too large (smaller terms start to vanish), so the
-// estimate is used for E <= 10.5 after lowering it by max(0, E - 6): the largest exponential of a
-// row then lies in [2^-6, 2^15]. Otherwise (or when a value exceeds e4m3's largest, 448, or is not
-// a number) gate[0] = 1 and the row maxima come from the half operands, exactly. The decision is a
-// function of the data only, so repeated runs take the same route. gate[1] receives the amount (in
-// raw score units, as float bits) by which the exp epilogue lowers the maxima it subtracts.
-__global__ void wide_gate_kernel(const unsigned int* __restrict__ stats_q, const unsigned int* __restrict__ stats_k,
-                                 int head_dim, float exp_scale, unsigned int* __restrict__ gate) {
-  const float nq = sqrtf(__uint_as_float(stats_q[0])), nk = sqrtf(__uint_as_float(stats_k[0]));
-  const float aq = __uint_as_float(stats_q[1]), ak = __uint_as_float(stats_k[1]);
-  const float e = 0.0625f, d = 0.0009765625f, n = static_cast<float>(head_dim);
-  const float err = (2.0f * e + e * e) * nq * nk + d * (nq + nk) * sqrtf(n) + n * d * d;
-  const float bound = err * exp_scale;
-  const bool safe = (aq <= 448.0f) && (ak <= 448.0f) && (bound <= 10.5f);  // false for NaN
-  gate[0] = safe ? 0u : 1u;
-  gate[1] = __float_as_uint(safe ? fmaxf(bound - 6.0f, 0.0f) / exp_scale : 0.0f);
-}
-
-// One warp per row: lane l adds partial[l], partial[l + 32], ... in order, then the lanes are
-// folded by xor shuffles: the same order on every run.
-__global__ void __launch_bounds__(256) row_sum_inverse_kernel(const float* __restrict__ partial, int n_partial,
-                                                              long long rows, float* __restrict__ inv) {
-  const long long row = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
-  if (row >= rows) return;
-  const int lane = threadIdx.x & 31;
-  float s = 0.0f;
-  for (int i = lane; i < n_partial; i += 32) s += partial[row * n_partial + i];
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
-  if (lane == 0) inv[row] = s > 0.0f ? 1.0f / s : 0.0f;  // an empty row yields zeros, not NaN
+  if (is_k) {
+    cast_block(a, a.k, static_cast<__half*>(a.k16), block - row_blocks, block_stats, false);
+  } else {
+    cast_block(a, a.q, static_cast<__half*>(a.q16), block, block_stats, a.zero != nullptr);
+    const int row = block * kRowsPerBlock + static_cast<int>(threadIdx.x);
+    if (threadIdx.x < kRowsPerBlock && row < a.tokens) {
+      a.row_key[row] = 0u;  // lies below the key of every float
+      if (row % 256 == 0) a.block_flags[row / 256] = 0u;
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    unsigned int* stats = a.state + (is_k ? kWideStatK : kWideStatQ);
+    atomicMax(stats, block_stats[0]);
+    atomicMax(stats + 1, block_stats[1]);
+    __threadfence();
+    // Counts to 2 * row_blocks and starts over at zero with the last block, which finds every block's maxima.
+    if (atomicInc(a.state + kWideCounter, 2u * row_blocks - 1u) == 2u * row_blocks - 1u) {
+      __threadfence();
+      unsigned int s[4];
+      for (int i = 0; i < 4; ++i) s[i] = atomicExch(a.state + i, 0u);  // and leaves them ready for the next call
+      a.state[kWideRoute] = choose_route(s, a.ch, a.exp_scale);
+    }
+  }
 }
 
 }  // namespace
 
-cudaError_t launch_transpose_cast(cudaStream_t stream, const float* in, void* out_f16, int tokens, int ch) {
-  const dim3 grid((tokens + 31) / 32, (ch + 31) / 32);
-  transpose_cast_kernel<<<grid, 256, 0, stream>>>(in, static_cast<__half*>(out_f16), tokens, ch);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_cast_f32_to_f16_e4m3(cudaStream_t stream, const float* in, void* out_f16, void* out_e4m3, long long rows,
-                                        int ch, unsigned int* stats) {
-  if (rows <= 0) return cudaSuccess;
-  if (ch % 4 != 0) return cudaErrorInvalidValue;
-  cast_f32_to_f16_e4m3_kernel<<<static_cast<unsigned>((rows + 7) / 8), 256, 0, stream>>>(
-      in, static_cast<__half*>(out_f16), static_cast<uint8_t*>(out_e4m3), rows, ch, stats);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_wide_gate(cudaStream_t stream, const unsigned int* stats_q, const unsigned int* stats_k, int head_dim,
-                             float exp_scale, unsigned int* gate) {
-  wide_gate_kernel<<<1, 1, 0, stream>>>(stats_q, stats_k, head_dim, exp_scale, gate);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_row_sum_inverse(cudaStream_t stream, const float* partial, int n_partial, long long rows, float* inv) {
-  if (rows <= 0) return cudaSuccess;
-  row_sum_inverse_kernel<<<static_cast<unsigned>((rows + 7) / 8), 256, 0, stream>>>(partial, n_partial, rows, inv);
-  return cudaGetLastError();
+cudaError_t launch_wide_cast(cudaStream_t stream, const WideCast& args) {
+  const int row_blocks = (args.tokens + kRowsPerBlock - 1) / kRowsPerBlock;
+  const int v_blocks = ((args.tokens + kVTile - 1) / kVTile) * ((args.ch + kVTile - 1) / kVTile);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * row_blocks + v_blocks);
+  cfg.blockDim = dim3(256);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, wide_cast_kernel, args, row_blocks);
 }
 
 }  // namespace zdraw

@@ -195,7 +195,7 @@ pub extern fn zdraw_cuda_static_last_status(stream: ?*anyopaque, status: *u32) c
 // Debugging: pipeline clock stamps of one CTA into a device buffer of >= 1600 u64 words (null = off).
 pub extern fn zdraw_cuda_attn_set_trace(ctx: *anyopaque, device_words: ?*anyopaque, n_words: usize) c_int;
 pub extern fn zdraw_cuda_last_status(ctx: *anyopaque, stream: ?*anyopaque, status: *u32) c_int;
-// Route of the last wide attention call's row maxima: 0 = e4m3 estimate (proven bound), 1 = half operands.
+// Route of the last wide attention call's row maxima: 0 = a sample of the keys, 1 = all keys (every row or some).
 pub extern fn zdraw_cuda_wide_attention_route(ctx: *anyopaque, stream: ?*anyopaque, exact_row_max: *u32) c_int;
 // Self-test: bounded waits that run out after limit_ns (<= 100 ms) and set bit 8 of the status word.
 pub extern fn zdraw_cuda_selftest_wait_timeout(ctx: *anyopaque, stream: ?*anyopaque, limit_ns: u64) c_int;
