@@ -70,12 +70,29 @@ def _torch_dtype_code(t) -> int:
 
 
 def _ptr(x):
-    """Device pointer of a torch tensor / host pointer of a numpy array / None."""
+    """Device pointer of a torch tensor / host pointer of a numpy array / None, as the address that the declared
+    ``c_void_p`` arguments take (no ctypes object per tensor: a joint call passes eleven of them)."""
     if x is None:
         return None
     if isinstance(x, np.ndarray):
-        return x.ctypes.data_as(C.c_void_p)
-    return C.c_void_p(x.data_ptr())
+        return x.ctypes.data
+    return x.data_ptr()
+
+
+_cuda = None  # torch.cuda and its raw-stream getter, looked up once
+
+
+def _current_stream_ptr() -> int:
+    """Handle of the current device's current stream, without the ``torch.cuda.Stream`` object that
+    ``torch.cuda.current_stream()`` makes of it (3.6 us of a 19 us call)."""
+    global _cuda
+    if _cuda is None:
+        import torch
+
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)
+        _cuda = (torch.cuda.current_device, raw or (lambda index: torch.cuda.current_stream(index).cuda_stream))
+    current_device, raw_stream = _cuda
+    return raw_stream(current_device())
 
 
 class Context:
@@ -121,11 +138,7 @@ class Context:
 
     @staticmethod
     def _stream_ptr(stream):
-        if stream is None:
-            import torch
-
-            stream = torch.cuda.current_stream()
-        return C.c_void_p(stream.cuda_stream)
+        return _current_stream_ptr() if stream is None else stream.cuda_stream
 
     def last_status(self, stream=None) -> int:
         st = C.c_uint32(0)
