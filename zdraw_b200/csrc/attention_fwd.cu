@@ -783,7 +783,7 @@ attn_fwd_steps_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       mbar_init(bar(kS1BarVFull + s), 1);
       mbar_init(bar(kS1BarVEmpty + s), 1);
       mbar_init(bar(kS1BarSFull + s), 1);
-      for (int i = 0; i < kPieces; ++i) mbar_init(bar(kS1BarPFull + kPieces * s + i), kBM);
+      for (int i = 0; i < kPieces; ++i) mbar_init(bar(kS1BarPFull + kPieces * s + i), kBM / 32);
     }
     mbar_init(bar(kS1BarOFull), 1);
     mbar_init(bar(kS1BarDrain), 1);
@@ -1114,7 +1114,10 @@ attn_fwd_steps_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
           if (piece_end(i) == 2 * (ch + 1)) {
             tmem_wait_st();
             tc_fence_before();
-            mbar_arrive(bar(kS1BarPFull + kPieces * b + i));
+            // One arrival per warp: 128 serialise on the barrier's word, and with one tile per CTA nothing hides that
+            // (768 tokens x 24 heads 15.76 -> 15.50 us; the two-tile kernel is no faster for it).
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar(kS1BarPFull + kPieces * b + i));
           }
         }
       }
