@@ -25,20 +25,27 @@ struct PartSpec {
   uint32_t n_valid = 0;              // row max / exp: real columns (0 = all n); W then has n_valid rows
 };
 
-// What only the wide attention's launches say.
+// What the wide attention's launches say beyond the parameters of the entry points.
 struct WideSpec {
   uint32_t w_k_valid = 0;         // columns of W that exist when fewer than k (A has all k)
   unsigned int* route = nullptr;  // device-side choice of the work (linear.cuh)
   unsigned int* block_flags = nullptr;
   int run_when = 0;
   bool rows_first = false;        // tile order: across the column blocks of a row block first
+  bool early_dependents = false;  // (projections: true)
   int k_splits = 1;               // 2: C holds zeros and each tile's K is walked by two pairs (linear.cuh)
 };
+
+WideSpec projection() {
+  WideSpec s;
+  s.early_dependents = true;
+  return s;
+}
 
 // Shared body of zdraw_cuda_linear and zdraw_cuda_qkv_projection: validates, builds the tensor
 // maps and launches one kernel that computes every part from the same A.
 int run_linear(Ctx* cx, void* stream, const void* a, int n_parts, const PartSpec* parts, const float* rope_cos,
-               const float* rope_sin, const zdraw_cuda_linear_params* p, const WideSpec& wide = WideSpec()) {
+               const float* rope_sin, const zdraw_cuda_linear_params* p, const WideSpec& wide) {
   if (!p) return fail(cx, ZDRAW_CUDA_E_ARG, "params is null");
   if (p->reserved != 0 || p->m == 0 || p->n == 0 || p->k == 0) return fail(cx, ZDRAW_CUDA_E_ARG, "zero size or reserved != 0");
   if (p->c_dtype != ZDRAW_DTYPE_F16 && p->c_dtype != ZDRAW_DTYPE_F32) return fail(cx, ZDRAW_CUDA_E_ARG, "bad c_dtype");
@@ -75,6 +82,7 @@ int run_linear(Ctx* cx, void* stream, const void* a, int n_parts, const PartSpec
   la.run_when = wide.run_when;
   la.rows_first = wide.rows_first ? 1 : 0;
   la.k_splits = wide.k_splits;
+  la.early_dependents = wide.early_dependents ? 1 : 0;
   if (any_qk) {
     if (p->tokens == 0 || p->heads == 0 || p->m % p->tokens != 0 || p->n != p->heads * 128u || p->txt_tokens > p->tokens)
       return fail(cx, ZDRAW_CUDA_E_ARG, "qk epilogue needs m = images * tokens and n = heads * 128");
@@ -165,7 +173,7 @@ int zdraw_cuda_linear(void* ctx, void* stream, const void* a, const void* w, voi
   if (p->epilogue > 1) return fail(cx, ZDRAW_CUDA_E_ARG, "bad epilogue");
   if (p->epilogue == 1 && p->c_dtype != ZDRAW_DTYPE_F16) return fail(cx, ZDRAW_CUDA_E_ARG, "the qk epilogue writes f16");
   const PartSpec part = {w, c, p->epilogue, norm_w_txt, norm_w_img};
-  return run_linear(cx, stream, a, 1, &part, rope_cos, rope_sin, p);
+  return run_linear(cx, stream, a, 1, &part, rope_cos, rope_sin, p, projection());
 }
 
 int zdraw_cuda_wide_attention(void* ctx, void* stream, const float* q, const float* k, const float* v, float* o,
@@ -248,7 +256,7 @@ int zdraw_cuda_wide_attention(void* ctx, void* stream, const float* q, const flo
   part_s.n_partial = static_cast<int>(n_partial);
   part_s.exp_scale = cast.exp_scale;
   part_s.n_valid = static_cast<uint32_t>(n_sample);
-  if ((rc = run_linear(cx, stream, cx->wa_q16.p, 1, &part_s, nullptr, nullptr, &ps)) != 0) return rc;
+  if ((rc = run_linear(cx, stream, cx->wa_q16.p, 1, &part_s, nullptr, nullptr, &ps, WideSpec())) != 0) return rc;
   ps.n = static_cast<uint32_t>(n_pad);
   ps.ld_w = head_dim;
   part_s.n_valid = static_cast<uint32_t>(tokens);
@@ -307,7 +315,7 @@ int zdraw_cuda_qkv_projection(void* ctx, void* stream, const void* x, const void
   if (!p) return fail(cx, ZDRAW_CUDA_E_ARG, "params is null");
   if (p->epilogue != 1) return fail(cx, ZDRAW_CUDA_E_ARG, "the q/k/v projection takes epilogue = 1 (q and k get the prologue)");
   const PartSpec parts[3] = {{wq, q16, 1, q_w_txt, q_w_img}, {wk, k16, 1, k_w_txt, k_w_img}, {wv, v, 0, nullptr, nullptr}};
-  return run_linear(cx, stream, x, 3, parts, rope_cos, rope_sin, p);
+  return run_linear(cx, stream, x, 3, parts, rope_cos, rope_sin, p, projection());
 }
 
 }  // extern "C"

@@ -61,6 +61,7 @@ struct LinearArgs {
   unsigned int* route;
   unsigned int* block_flags;
   int run_when;
+  int early_dependents;  // 1: the next launch in the stream may be set up before this one ends
   // Tile order: 0 = down the rows of one column block (W stays in L2), 1 = across the column blocks
   // of one row block (A stays in L2).
   int rows_first;
