@@ -4,8 +4,8 @@
     python profile_case.py --workload klein_1024 --iters 4 --case linear_qk   (or linear_plain, wide)
     python profile_case.py --workload klein_1024 --iters 4 --heads 3          (a head shard: attn_fwd_steps_kernel)
 
-One untimed call, then `iters` timed ones. Launches per call: qk_norm_rope_kernel, attn_fwd_kernel (plus mask_prepare_kernel with a key
-mask and cast_f32_to_f16_kernel for f32 inputs). Prints the mean device time per iteration.
+One untimed call, then `iters` timed ones. Launches per call: qk_norm_rope_kernel (which also makes a key mask's
+tile lists and casts an f32 V), attn_fwd_kernel. Prints the mean device time per iteration.
 """
 from __future__ import annotations
 

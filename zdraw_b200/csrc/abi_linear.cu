@@ -237,7 +237,7 @@ int zdraw_cuda_wide_attention(void* ctx, void* stream, const float* q, const flo
   // exact maxima by two launches that otherwise leave at once, as is everything when the operands' norms are
   // too large for the sample to be worth trying (choose_route). All of it depends on the data alone. (The
   // reference takes the exact f32 maximum of half products, krow_softmax_h, src/metal/mvattn_owned.zig:95-128.)
-  // Together with the split P V and the one cast launch: 94 -> 63 us at 4096 x 512, 759 -> 626 us at 16384 x 512,
+  // Together with the split P V and the one cast launch: 94 -> 61 us at 4096 x 512, 759 -> 616 us at 16384 x 512,
   // against row maxima from e4m3 copies of all keys. A call whose every block is done again takes about as much
   // longer as one more exp product (26 and 275 us).
   // Below 1024 tokens every key is in the sample: its maxima are exact and nothing can need doing again.
