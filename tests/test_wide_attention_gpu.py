@@ -175,3 +175,37 @@ def test_keys_outside_the_sample_are_noticed(ctx, oracle, tokens):
     q2, k2, v2 = make(tokens, dim, tokens + 1)
     ctx.wide_attention(q2, k2, v2, out, cfg)
     assert ctx.wide_attention_route() == 0  # the next call starts afresh
+
+
+@pytest.mark.parametrize("tokens", [1056, 2080])
+def test_norms_decide_how_row_maxima_are_taken(ctx, oracle, tokens):
+    """Above 1024 tokens, last row block ragged: a dominant key outside the sample (every 2nd, every 4th key) with a value
+    of 500, under norms that allow scores of 600, takes the maxima of all keys; the same value with norms that keep every
+    score below 80 does not; a NaN does, and the rows it is not in come out right. None of it reaches the next call."""
+    dim = 512
+    cfg = mattn.Config(tokens, 1, 1, dim)
+    q, k, v = make(tokens, dim, 11, scale=0.05)
+    out = torch.full((tokens, dim), float("nan"), device="cuda")
+
+    def check(rows, route):
+        ctx.wide_attention(q, k, v, out, cfg)
+        torch.cuda.synchronize()
+        assert ctx.wide_attention_route() == route and ctx.last_status() == 0
+        qh, kh = q.half().float().cpu().numpy(), k.half().float().cpu().numpy()
+        for r in rows:
+            want = oracle.sdpa(qh, kh, v.cpu().numpy(), heads=1, rows=(r, r + 1)).reshape(tokens, dim)[r]
+            err = np.abs(out[r].cpu().numpy() - want)
+            assert err.max() <= 2e-2 and err.mean() <= 2e-3, f"row {r}: {err.max()}"
+
+    k[7], k[9] = 0.0, 0.0
+    k[7, 0], k[9, 0] = 500.0, 470.0  # key 7 wins by 30 * 20 / sqrt(512) = 26
+    q[:, 0] = 20.0
+    check((0, 255, 256, 1030, tokens - 1), 1)
+    assert np.allclose(out.cpu().numpy(), v[7].half().float().cpu().numpy()[None, :], atol=2e-3)
+    q[:, 0] = 0.0  # |q| = 1.2, |k| = 500
+    check((0, 256, tokens - 1), 0)
+    k[7], k[9] = k[8], k[8]
+    q[40, 3] = float("nan")
+    check((0, 39, 41, tokens - 1), 1)
+    q[40, 3] = 0.0
+    check((0, 40, tokens - 1), 0)

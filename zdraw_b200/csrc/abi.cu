@@ -361,8 +361,8 @@ int zdraw_cuda_attn_create(int device, void** ctx_out) {
     return ZDRAW_CUDA_E_CUDA;
   }
   c->encode = reinterpret_cast<EncodeTiledFn>(fn);
-  if (cudaMalloc(reinterpret_cast<void**>(&c->d_status), 256) != cudaSuccess ||
-      cudaMemset(c->d_status, 0, 256) != cudaSuccess ||
+  if (cudaMalloc(reinterpret_cast<void**>(&c->d_status), kStatusBytes) != cudaSuccess ||
+      cudaMemset(c->d_status, 0, kStatusBytes) != cudaSuccess ||
       cudaStreamCreateWithFlags(&c->host_stream, cudaStreamNonBlocking) != cudaSuccess ||
       zdraw::attn_fwd_configure() != cudaSuccess || zdraw::linear_configure() != cudaSuccess) {
     if (c->d_status) cudaFree(c->d_status);
@@ -370,7 +370,7 @@ int zdraw_cuda_attn_create(int device, void** ctx_out) {
     delete c;
     return ZDRAW_CUDA_E_CUDA;
   }
-  c->wa_state = c->d_status + 32;  // zeroed with the status word
+  c->wa_state = c->d_status + kWideStateAt;  // zeroed with the status word
   *ctx_out = c;
   return ZDRAW_CUDA_OK;
 }

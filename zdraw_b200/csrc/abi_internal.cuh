@@ -10,12 +10,17 @@
 #include <cstdio>
 
 #include "../../include/zdraw_cuda.h"
+#include "wide_attention.cuh"
 
 namespace zdraw {
 namespace abi {
 
 
 constexpr int kHeadDim = 128;
+// The context's status allocation: the status word, and on a line of their own the words of the wide attention.
+constexpr size_t kStatusBytes = 256;
+constexpr int kWideStateAt = 32;
+static_assert((kWideStateAt + kWideStateWords) * sizeof(uint32_t) <= kStatusBytes, "words of the status allocation");
 constexpr uint32_t kMaxTokens = 1u << 20;
 constexpr float kLog2e = 1.4426950408889634f;
 
@@ -46,7 +51,7 @@ struct Ctx {
   Buf q16, k16, v16, tile_list;
   Buf st_q, st_k, st_v, st_o, st_w, st_cos, st_sin, st_mask;  // staging for the host-buffer path
   Buf wa_q16, wa_k16, wa_vt16, wa_aux, wa_p;  // wide-head attention: half operands, row statistics, exp(scores)
-  unsigned int* wa_state = nullptr;            // kWideStateWords words behind d_status (wide_attention.cuh)
+  unsigned int* wa_state = nullptr;            // the words of wide_attention.cuh, at d_status + kWideStateAt
   bool wa_ran = false;                         // a wide attention call has been made
   // Device-resident RoPE tables for the host-buffer joint call (zdraw_cuda_attn_set_device_tables).
   const float* dev_cos = nullptr;

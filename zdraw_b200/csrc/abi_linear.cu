@@ -28,8 +28,10 @@ struct PartSpec {
 // What the wide attention's launches say beyond the parameters of the entry points.
 struct WideSpec {
   uint32_t w_k_valid = 0;         // columns of W that exist when fewer than k (A has all k)
-  unsigned int* route = nullptr;  // device-side choice of the work (linear.cuh)
-  unsigned int* block_flags = nullptr;
+  const unsigned int* norms = nullptr;  // row max: see LinearArgs; all of W is n_valid_all rows of k
+  uint32_t n_valid_all = 0;
+  unsigned int *all_rows = nullptr, *norms_done = nullptr;
+  unsigned int *missed = nullptr, *block_flags = nullptr;  // blocks to be done again (linear.cuh)
   int run_when = 0;
   bool rows_first = false;        // tile order: across the column blocks of a row block first
   bool early_dependents = false;  // (projections: true)
@@ -77,7 +79,13 @@ int run_linear(Ctx* cx, void* stream, const void* a, int n_parts, const PartSpec
   la.k = static_cast<int>(p->k);
   la.n_parts = n_parts;
   la.status = cx->d_status;
-  la.route = wide.route;
+  la.norms = wide.norms;
+  la.norm_scale = parts[0].exp_scale;
+  la.n_valid_all = static_cast<int>(wide.n_valid_all);
+  la.n_all = (la.n_valid_all + 255) / 256 * 256;
+  la.all_rows = wide.all_rows;
+  la.norms_done = wide.norms_done;
+  la.missed = wide.missed;
   la.block_flags = wide.block_flags;
   la.run_when = wide.run_when;
   la.rows_first = wide.rows_first ? 1 : 0;
@@ -142,6 +150,8 @@ int run_linear(Ctx* cx, void* stream, const void* a, int n_parts, const PartSpec
         CUDA_SUCCESS)
       return fail(cx, ZDRAW_CUDA_E_CUDA, "cuTensorMapEncodeTiled failed");
   }
+  if (wide.norms && encode(&maps.w[1], parts[0].w, wide.n_valid_all, p->k, p->k) != CUDA_SUCCESS)
+    return fail(cx, ZDRAW_CUDA_E_CUDA, "cuTensorMapEncodeTiled failed");
   // Plain parts: C for the epilogue's tile stores (32 columns x 32 rows, swizzle of the row size).
   for (int i = 0; i < zdraw::kMaxLinearParts; ++i) {
     maps.c[i] = maps.a;  // any valid map where none is used
@@ -212,7 +222,6 @@ int zdraw_cuda_wide_attention(void* ctx, void* stream, const float* q, const flo
   cast.vt16 = cx->wa_vt16.p;
   cast.tokens = static_cast<int>(tokens);
   cast.ch = static_cast<int>(head_dim);
-  cast.exp_scale = 1.4426950408889634f / std::sqrt(static_cast<float>(head_dim));
   cast.row_key = row_key;
   cast.block_flags = block_flags;
   cast.state = cx->wa_state;
@@ -234,12 +243,13 @@ int zdraw_cuda_wide_attention(void* ctx, void* stream, const float* q, const flo
   // overflows, so the maxima come from some 512 keys spread over the image (every stride-th one, through
   // the tensor map's row stride). A row whose largest score lies more than 2^16 above the sample's
   // (in the exponentials) is noticed by the exp product; its block of 256 rows is then done again from the
-  // exact maxima by two launches that otherwise leave at once, as is everything when the operands' norms are
-  // too large for the sample to be worth trying (choose_route). All of it depends on the data alone. (The
+  // exact maxima by two launches that otherwise leave at once. Operands of large norms (scores beyond
+  // kMaxSampledScore possible) get the maxima of all keys from the first launch: nearly every block would be
+  // done again. All of it depends on the data alone. (The
   // reference takes the exact f32 maximum of half products, krow_softmax_h, src/metal/mvattn_owned.zig:95-128.)
   // Together with the split P V and the one cast launch: 94 -> 61 us at 4096 x 512, 759 -> 616 us at 16384 x 512,
-  // against row maxima from e4m3 copies of all keys. A call whose every block is done again takes about as much
-  // longer as one more exp product (26 and 275 us).
+  // against row maxima from e4m3 copies of all keys. A call whose every block is done again multiplies Q by all keys
+  // twice more: 99 us instead of 61 and 1090 instead of 530 (of the same inputs' times after an idle second).
   // Below 1024 tokens every key is in the sample: its maxima are exact and nothing can need doing again.
   const size_t stride = tokens < 1024 ? 1 : tokens / 512;
   const size_t n_sample = (tokens + stride - 1) / stride;
@@ -254,16 +264,21 @@ int zdraw_cuda_wide_attention(void* ctx, void* stream, const float* q, const flo
   part_s.row_key = row_key;
   part_s.row_sum = row_sum;
   part_s.n_partial = static_cast<int>(n_partial);
-  part_s.exp_scale = cast.exp_scale;
+  part_s.exp_scale = 1.4426950408889634f / std::sqrt(static_cast<float>(head_dim));
   part_s.n_valid = static_cast<uint32_t>(n_sample);
-  if ((rc = run_linear(cx, stream, cx->wa_q16.p, 1, &part_s, nullptr, nullptr, &ps, WideSpec())) != 0) return rc;
+  WideSpec max_spec;
+  max_spec.norms = cx->wa_state + zdraw::kWideNorms;
+  max_spec.n_valid_all = static_cast<uint32_t>(tokens);
+  max_spec.all_rows = cx->wa_state + zdraw::kWideAllKeys;
+  if ((rc = run_linear(cx, stream, cx->wa_q16.p, 1, &part_s, nullptr, nullptr, &ps, max_spec)) != 0) return rc;
   ps.n = static_cast<uint32_t>(n_pad);
   ps.ld_w = head_dim;
   part_s.n_valid = static_cast<uint32_t>(tokens);
   WideSpec when;
-  when.block_flags = block_flags;
+  when.norms_done = cx->wa_state + zdraw::kWideNorms;
   if (stride > 1) {
-    when.route = cx->wa_state + zdraw::kWideRoute;
+    when.missed = cx->wa_state + zdraw::kWideMissed;
+    when.block_flags = block_flags;
     when.run_when = zdraw::kRunEstimate;
   }
   part_s.epilogue = static_cast<uint32_t>(zdraw::kEpilogueExp);
@@ -300,9 +315,9 @@ int zdraw_cuda_wide_attention_route(void* ctx, void* stream, uint32_t* exact_row
   if (!cx->wa_ran) return fail(cx, ZDRAW_CUDA_E_ARG, "no wide attention call has run on this context");
   ZD_CUDA(cx, cudaSetDevice(cx->device));
   ZD_CUDA(cx, cudaStreamSynchronize(static_cast<cudaStream_t>(stream)));
-  uint32_t route = 0;
-  ZD_CUDA(cx, cudaMemcpy(&route, cx->wa_state + zdraw::kWideRoute, sizeof(route), cudaMemcpyDeviceToHost));
-  *exact_row_max = route != 0 ? 1u : 0u;
+  uint32_t state[zdraw::kWideStateWords] = {};
+  ZD_CUDA(cx, cudaMemcpy(state, cx->wa_state, sizeof(state), cudaMemcpyDeviceToHost));
+  *exact_row_max = state[zdraw::kWideAllKeys] | state[zdraw::kWideMissed];
   return ZDRAW_CUDA_OK;
 }
 

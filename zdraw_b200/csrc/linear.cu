@@ -100,12 +100,10 @@ __device__ __forceinline__ uint32_t pack_clamped(float lo, float hi) {
 __global__ void __launch_bounds__(kThreads, 1)
 linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  if (a.route != nullptr) {
-    // A launch of the wide attention that may have nothing to do leaves before it sets anything up
-    // (both CTAs of a pair see the same word: it changes between 0 and 2 only while run_when is kRunEstimate).
+  if (a.run_when == kRunExact) {
+    // A launch of the wide attention that may have nothing to do leaves before it sets anything up.
     grid_dependency_wait();
-    const unsigned int route = ld_volatile_u32(a.route);
-    if (a.run_when == kRunEstimate ? route == 1u : route == 0u) return;
+    if (ld_volatile_u32(a.missed) == 0u) return;
   }
   const uint32_t base = smem_u32(smem_raw);
   volatile uint32_t* flags = reinterpret_cast<volatile uint32_t*>(smem_raw + kOffFlags);
@@ -116,11 +114,7 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_cta_rank();  // 0: issues the pair's MMAs
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
-  const int tiles_n = (a.n + kTN - 1) / kTN;            // column blocks of one part (the last may be partial)
   const int tiles_m = (a.m + 2 * kTM - 1) / (2 * kTM);  // pair tiles: 256 rows
-  // With k_splits == 2 a tile of C is computed twice, by neighbouring work items that each walk half of K
-  // and add their share to C.
-  const int n_items = tiles_m * tiles_n * a.n_parts * a.k_splits;
   // A stage is a 128-byte slice of K per row; rows, columns and K beyond the matrices read as zeros.
   const int k_steps_all = (a.k + kTK - 1) / kTK;
   auto first_k = [&](int item) { return (item % a.k_splits) * (k_steps_all / a.k_splits); };
@@ -162,9 +156,21 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
   // The kernel behind a projection may set itself up on SMs that run out of work (sub-block at 512 pixels 141.2 us
   // without, 138.9 with). Not between the wide attention's launches (4096 x 512: 61.7 us without, 62.7 with).
   if (a.early_dependents) grid_launch_dependents();
+  // Both CTAs of a pair and every role see the same norms: the launch before this one wrote them.
+  const bool all_rows = a.norms != nullptr &&
+                        !(sqrtf(__uint_as_float(ld_volatile_u32(a.norms))) * sqrtf(__uint_as_float(ld_volatile_u32(a.norms + 1))) *
+                              a.norm_scale <= kMaxSampledScore);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (all_rows) *a.all_rows = 1u;
+    if (a.norms_done != nullptr) a.norms_done[0] = a.norms_done[1] = 0u;
+  }
+  const int tiles_n = ((all_rows ? a.n_all : a.n) + kTN - 1) / kTN;  // column blocks of one part (the last may be partial)
+  // With k_splits == 2 a tile of C is computed twice, by neighbouring work items that each walk half of K
+  // and add their share to C.
+  const int n_items = tiles_m * tiles_n * a.n_parts * a.k_splits;
   // When only some row blocks are to be done again, the others' tiles are passed over by every role alike.
   const unsigned int* const block_flags =
-      (a.route != nullptr && a.run_when == kRunExact && ld_volatile_u32(a.route) == 2u) ? a.block_flags : nullptr;
+      a.run_when == kRunExact ? a.block_flags : nullptr;
   auto passed_over = [&](int tile_m) -> bool { return block_flags != nullptr && ld_volatile_u32(block_flags + tile_m) == 0u; };
 
   if (warp == 0) {
@@ -185,7 +191,7 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
         const int tile_m = a.rows_first ? tile / n_cols : tile % tiles_m;
         if (passed_over(tile_m)) continue;
         const int tile_n = col % tiles_n;
-        const CUtensorMap* tm_w = &maps.w[col / tiles_n];
+        const CUtensorMap* tm_w = &maps.w[all_rows ? 1 : col / tiles_n];
         const int row_a = (2 * tile_m + static_cast<int>(rank)) * kTM;
         const int row_w = tile_n * kTN + static_cast<int>(rank) * (kTN / 2);
         for (int ks = first_k(item), ke = end_k(item); ks < ke; ++ks, ++it) {
@@ -295,6 +301,7 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
 
       if (part.epilogue == kEpilogueRowMax) {
         // Row maximum of the tile's columns, nothing stored: each thread reduces its 128 columns.
+        const int n_valid = all_rows ? a.n_valid_all : part.n_valid;
         float mx = -INFINITY;
 #pragma unroll 1
         for (int pc = 0; pc < 4; ++pc) {
@@ -302,13 +309,13 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
           tmem_ld_x32(t_acc + 32u * pc, x);
           tmem_wait_ld();
           const int col0 = 128 * half_n + 32 * pc;
-          if (col0 + 32 <= part.n_valid) {
+          if (col0 + 32 <= n_valid) {
 #pragma unroll
             for (int i = 0; i < 32; i += 2) mx = max3(mx, __uint_as_float(x[i]), __uint_as_float(x[i + 1]));
           } else {  // the ragged end of the row (at most once per row)
 #pragma unroll
             for (int i = 0; i < 32; ++i)
-              if (col0 + i < part.n_valid) mx = fmaxf(mx, __uint_as_float(x[i]));
+              if (col0 + i < n_valid) mx = fmaxf(mx, __uint_as_float(x[i]));
           }
         }
         if (live) atomicMax(part.row_key + m, float_key(mx));
@@ -445,7 +452,7 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
           if (top > -INFINITY && !(fmaf(top, mul, bias) < 15.99f)) {
             if (a.run_when == kRunEstimate) {  // a key outside the sample lies more than 2^16 above it
               a.block_flags[pair_m] = 1u;
-              *a.route = 2u;
+              *a.missed = 1u;
             } else {
               atomicOr(a.status, kStExpClamp);
             }
@@ -612,7 +619,7 @@ cudaError_t linear_pairs(int sm_count, int* out) {
 }
 
 cudaError_t launch_linear(cudaStream_t stream, const LinearMaps& maps, const LinearArgs& args, int pairs) {
-  const int n_tiles = linear_tiles(args.m, args.n, args.n_parts) * args.k_splits;
+  const int n_tiles = linear_tiles(args.m, args.norms != nullptr ? args.n_all : args.n, args.n_parts) * args.k_splits;
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[2];
   launch_config(&cfg, attr, stream);

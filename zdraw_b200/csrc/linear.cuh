@@ -14,6 +14,9 @@ constexpr int kEpilogueExp = 3;     // C = half(exp2((A W^T - max[row]) * exp_sc
 
 constexpr int kRunEstimate = 1, kRunExact = 2;  // LinearArgs::run_when
 
+// Largest score (in exp2 units) up to which row maxima are taken from a sample, see LinearArgs::norms.
+constexpr float kMaxSampledScore = 80.0f;
+
 constexpr int kMaxLinearParts = 3;
 
 // One output of a launch: C_p[m, n] = A[m, k] * W_p[n, k]^T with its own epilogue.
@@ -53,12 +56,18 @@ struct LinearArgs {
   const float *rope_cos, *rope_sin;  // [tokens][128]
   long long rope_batch_stride;
   uint32_t* status;
-  // Launches of the wide attention that a word in device memory decides on (nullptr: always runs).
-  // *route is 0 (row maxima come from a sample of the keys), 1 (exact maxima for every row) or 2 (exact
-  // maxima for the blocks of 256 rows whose flag is set: a score left the half range). A kRunEstimate launch
-  // leaves at once when it is 1, and its exp epilogue sets the flags and the 2; a kRunExact launch
-  // leaves at once when it is 0 and passes over the blocks that are not flagged when it is 2.
-  unsigned int* route;
+  // Row max over a sample of the rows of W (the wide attention): norms holds the largest |row|^2 of A and of the whole W
+  // as float bits, and where |row of A| |row of W| norm_scale can exceed kMaxSampledScore (or is not a number) the
+  // launch takes all of W instead: n_all columns, n_valid_all of them real, through maps.w[1]; *all_rows is set to 1.
+  const unsigned int* norms;
+  float norm_scale;
+  int n_all, n_valid_all;
+  unsigned int* all_rows;
+  unsigned int* norms_done;  // exp: two words that the launch leaves at zero (the norms, for the call after this one)
+  // Blocks of 256 rows that the wide attention does again (missed == nullptr: no such launch). The exp epilogue of a
+  // kRunEstimate launch flags the blocks where a score left the half range and sets *missed; a kRunExact launch
+  // leaves at once when *missed is 0 and passes over the blocks that are not flagged.
+  unsigned int* missed;
   unsigned int* block_flags;
   int run_when;
   int early_dependents;  // 1: the next launch in the stream may be set up before this one ends

@@ -3,7 +3,7 @@
 // half Q, K and V^T, S = Q K^T with f32 output, a row softmax writing half P, O = P (V^T)^T), with
 // the softmax (krow_softmax_h, :95-128) folded into the epilogues of linear_kernel so that the f32
 // scores never reach memory. This file holds the casts of Q and K (kf32_to_h), the transpose-and-cast
-// of V (kvt_transpose_h, :84-94) and the choice of how the row maxima are taken.
+// of V (kvt_transpose_h, :84-94) and the operands' norms, by which the row maxima are taken.
 #include "wide_attention.cuh"
 
 #include <cuda_fp16.h>
@@ -47,13 +47,11 @@ __device__ __forceinline__ void transpose_block(const WideCast& a, int block, __
   }
 }
 
-// Q or K: one warp per row, four floats per lane and step -> four halves (clamped). The warp also takes
-// the row's sum of squares (each lane adds its elements in order, the lanes are folded by xor shuffles:
-// the same order on every run) and its largest magnitude; the block's maxima end in block_stats as float
-// bits (non-negative floats order like unsigned integers, and a maximum does not depend on the order of
-// the updates). NaN inputs set block_stats[1] to the NaN pattern.
-__device__ __forceinline__ void cast_block(const WideCast& a, const float* in, __half* out16, int block,
-                                           unsigned int* block_stats, bool zero_rows) {
+// Q or K: one warp per row, four floats per lane and step -> four halves (clamped). The block's largest row sum of
+// squares raises *norm as float bits (which order like unsigned integers; a NaN lies above them all), so the
+// result does not depend on the order of the updates.
+__device__ __forceinline__ void cast_block(const WideCast& a, const float* in, __half* out16, int block, bool zero_rows,
+                                           unsigned int* block_norm, unsigned int* norm) {
   const int row_raw = block * kRowsPerBlock + (static_cast<int>(threadIdx.x) >> 5);
   const bool live = row_raw < a.tokens;
   const long long row = live ? row_raw : a.tokens - 1;  // a repeated row changes no maximum and is not stored
@@ -61,8 +59,7 @@ __device__ __forceinline__ void cast_block(const WideCast& a, const float* in, _
   const float4* src = reinterpret_cast<const float4*>(in + row * a.ch);
   uint2* dst16 = reinterpret_cast<uint2*>(out16 + row * a.ch);
   float4* zero = zero_rows ? reinterpret_cast<float4*>(a.zero + row * a.ch) : nullptr;
-  float ss = 0.0f, amax = 0.0f;
-  bool bad = false;
+  float ss = 0.0f;
   const int n4 = a.ch / 4;
   // Four loads in flight per lane (512 floats per pass of the warp): the row of the VAE shape in one pass.
   for (int i0 = lane; i0 < n4; i0 += 128) {
@@ -79,8 +76,6 @@ __device__ __forceinline__ void cast_block(const WideCast& a, const float* in, _
       ss = fmaf(v.y, v.y, ss);
       ss = fmaf(v.z, v.z, ss);
       ss = fmaf(v.w, v.w, ss);
-      amax = fmaxf(fmaxf(amax, fmaxf(fabsf(v.x), fabsf(v.y))), fmaxf(fabsf(v.z), fabsf(v.w)));
-      bad = bad || !(v.x == v.x) || !(v.y == v.y) || !(v.z == v.z) || !(v.w == v.w);
       const __half2 h0 = __floats2half2_rn(clamp_half(v.x), clamp_half(v.y));
       const __half2 h1 = __floats2half2_rn(clamp_half(v.z), clamp_half(v.w));
       uint2 o;
@@ -91,70 +86,35 @@ __device__ __forceinline__ void cast_block(const WideCast& a, const float* in, _
     }
   }
 #pragma unroll
-  for (int off = 16; off > 0; off >>= 1) {
-    ss += __shfl_xor_sync(0xffffffffu, ss, off);
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
-  }
-  bad = __any_sync(0xffffffffu, bad);
-  if (lane == 0) {
-    atomicMax(block_stats + 0, __float_as_uint(ss));  // +inf orders above every finite value
-    atomicMax(block_stats + 1, bad ? 0x7fc00000u : __float_as_uint(amax));
-  }
+  for (int off = 16; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+  if (threadIdx.x == 0) *block_norm = 0u;
+  __syncthreads();
+  if (lane == 0) atomicMax(block_norm, __float_as_uint(ss));
+  __syncthreads();
+  if (threadIdx.x == 0) atomicMax(norm, *block_norm);
 }
 
-// Whether the row maxima may come from a sample of the keys, from the operands' statistics alone. A
-// sampled maximum is never above the true one, so the largest exponential of a row is at least 1, and it
-// fits half as long as the true maximum lies less than 2^16 above the sampled one in the exponentials.
-// The exp product notices a row where it does not, and its block of 256 rows is done again from the exact maxima:
-// that costs a block as much as the exact route from the beginning plus the lost product, so the sample is only
-// tried while scores are moderate: largest norms |q| |k| * scale (which bounds every score) up to 81 in
-// units of the exponent, no value beyond 448, no NaN. (N(0,1) operands at 512 channels: 42.)
-__device__ __forceinline__ unsigned int choose_route(const unsigned int* stats, int ch, float exp_scale) {
-  const float nq = sqrtf(__uint_as_float(stats[kWideStatQ])), nk = sqrtf(__uint_as_float(stats[kWideStatK]));
-  const float aq = __uint_as_float(stats[kWideStatQ + 1]), ak = __uint_as_float(stats[kWideStatK + 1]);
-  const float e = 0.0625f, d = 0.0009765625f, n = static_cast<float>(ch);
-  const float spread = (2.0f * e + e * e) * nq * nk + d * (nq + nk) * sqrtf(n) + n * d * d;
-  return (aq <= 448.0f && ak <= 448.0f && spread * exp_scale <= 10.5f) ? 0u : 1u;  // 1 for NaN
-}
-
-// One launch for the three operands (three launches, two memsets and a one-thread kernel for the route took
-// about 25 us of a call at 4096 x 512, this takes 8). Memory-bound: 6 bytes per element, 26 us at 16384 x 512.
+// One launch for the three operands (three launches, two memsets and a one-thread kernel took about 25 us of a
+// call at 4096 x 512, this takes 8). Memory-bound: 6 bytes per element, 26 us at 16384 x 512.
 __global__ void __launch_bounds__(256) wide_cast_kernel(const WideCast a, int row_blocks) {
   __shared__ __half tile[kVTile][kVTile + 2];
-  __shared__ unsigned int block_stats[2];
+  __shared__ unsigned int block_norm;
   // The launches before this one may still read what it writes.
   grid_dependency_wait();
   grid_launch_dependents();
   const int block = static_cast<int>(blockIdx.x);
   if (block >= 2 * row_blocks) {
     transpose_block(a, block - 2 * row_blocks, tile);
-    return;
-  }
-  const bool is_k = block >= row_blocks;
-  if (threadIdx.x < 2) block_stats[threadIdx.x] = 0u;
-  __syncthreads();
-  if (is_k) {
-    cast_block(a, a.k, static_cast<__half*>(a.k16), block - row_blocks, block_stats, false);
+  } else if (block >= row_blocks) {
+    cast_block(a, a.k, static_cast<__half*>(a.k16), block - row_blocks, false, &block_norm,
+               a.state + kWideNorms + 1);
   } else {
-    cast_block(a, a.q, static_cast<__half*>(a.q16), block, block_stats, a.zero != nullptr);
+    cast_block(a, a.q, static_cast<__half*>(a.q16), block, a.zero != nullptr, &block_norm, a.state + kWideNorms);
     const int row = block * kRowsPerBlock + static_cast<int>(threadIdx.x);
     if (threadIdx.x < kRowsPerBlock && row < a.tokens) {
       a.row_key[row] = 0u;  // lies below the key of every float
       if (row % 256 == 0) a.block_flags[row / 256] = 0u;
-    }
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned int* stats = a.state + (is_k ? kWideStatK : kWideStatQ);
-    atomicMax(stats, block_stats[0]);
-    atomicMax(stats + 1, block_stats[1]);
-    __threadfence();
-    // Counts to 2 * row_blocks and starts over at zero with the last block, which finds every block's maxima.
-    if (atomicInc(a.state + kWideCounter, 2u * row_blocks - 1u) == 2u * row_blocks - 1u) {
-      __threadfence();
-      unsigned int s[4];
-      for (int i = 0; i < 4; ++i) s[i] = atomicExch(a.state + i, 0u);  // and leaves them ready for the next call
-      a.state[kWideRoute] = choose_route(s, a.ch, a.exp_scale);
+      if (row == 0) a.state[kWideAllKeys] = a.state[kWideMissed] = 0u;
     }
   }
 }
