@@ -634,7 +634,7 @@ def main():
         wide = {"api": "zdraw_cuda_wide_attention", "tokens": wt, "head_dim": wd, "ms_per_call": ms_w, "idle_before_s": 1.0,
                 "achieved": 4.0 * wt * wt * wd / ms_w / 1e9, "unit": "TFLOP/s",
                 "kernels": "wide_cast_kernel (q, k, v to half, v transposed), linear_kernel x3 (row maxima over a sample of the keys; "
-                           "exp(S - max) in half + row sums; P V / row sum), and two that leave at once",
+                           "exp(S - max) in half + row sums; P V / row sum), wide_rescale_kernel (leaves at once)",
                 "l2": "exp(scores) in half (0.5 GB) streams through HBM once each way"}
         del wq, wk, wv, wo
         if ctx.last_status() != 0:

@@ -418,9 +418,9 @@ ZDRAW_CUDA_API int zdraw_cuda_wide_attention(void *ctx, void *stream, const floa
 
 /*
  * Which way the last zdraw_cuda_wide_attention call on this context took its row maxima: 0 = from a
- * sample of the keys, for every row (tried when the operands' norms keep the scores moderate; no row's
- * maximum lay more than 2^16 above its sample in the exponentials), 1 = from all keys (the reference's
- * exact form), for every row or for the blocks of 256 rows where the sample had missed it. Below 1024 tokens every
+ * sample of the keys, for every row (when the operands' norms keep the scores moderate; no row's
+ * maximum lay 2^16 or more above its sample in the exponentials), 1 = from all keys, for every row (the
+ * reference's exact form) or for the rows where the sample had missed it, which are rescaled. Below 1024 tokens every
  * key is in the sample, and the value only says whether the norms would have called for all keys. The choice is
  * made on the device from the data alone, so repeats take the same route. Plays the part of the bridge's per-route counters (metal_api.m:350, 459). Synchronises
  * `stream`.

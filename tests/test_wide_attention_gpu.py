@@ -147,8 +147,8 @@ def test_shapes_outside_the_kernels_are_declined(ctx):
 @pytest.mark.parametrize("tokens", [1024, 1056, 2080, 4096])
 def test_keys_outside_the_sample_are_noticed(ctx, oracle, tokens):
     """Row maxima come from every (tokens // 512)-th key; a key outside that sample that equals a query of usual norm
-    lies e^15 above the rest (512 / sqrt(512) = 22.6), beyond what the half range holds: that block of 256 rows (and
-    the last, ragged one) is done again from exact maxima, the others are not, and every row matches the oracle."""
+    lies e^15 above the rest (512 / sqrt(512) = 22.6), beyond what the half range holds: that row (and one of the last,
+    ragged block) is rescaled, the others are not, and every row matches the oracle."""
     dim = 512
     q, k, v = make(tokens, dim, tokens)
     hits = {301: 7, tokens - 1: tokens - 3}  # row -> key, no multiple of the stride (2, 2, 4, 8)
@@ -209,3 +209,97 @@ def test_norms_decide_how_row_maxima_are_taken(ctx, oracle, tokens):
     check((0, 39, 41, tokens - 1), 1)
     q[40, 3] = 0.0
     check((0, 40, tokens - 1), 0)
+
+
+def missed(tokens, dim, seed, rows):
+    """N(0, 1) operands; keys outside the sample hold multiples of the given rows' queries, three to a row in different
+    blocks of 128 keys: scores of about 14, 18 and 22 (20, 26 and 32 in the exponent of 2), above some 3 of the sample."""
+    q, k, v = make(tokens, dim, seed)
+    stride = tokens // 512
+    free = [j for j in range(tokens) if j % stride]
+    for n, r in enumerate(rows):
+        for i, f in enumerate((0.62, 0.8, 0.97)):
+            k[free[(5 * n + 11 + i * (len(free) // 3)) % len(free)]] = q[r] * f
+    return q, k, v
+
+
+@pytest.mark.parametrize("tokens,n_rows", [(1024, 1), (1056, 60), (2080, 40), (3008, 100), (4096, 100)])
+def test_rows_the_sample_missed(ctx, tokens, n_rows):
+    """Rows with pieces at up to four scales (and their neighbours that have none), the last row block and the last block
+    of keys ragged, against float64 on the half operands."""
+    dim = 512
+    rows = sorted({(i * 7919 + 3) % tokens for i in range(n_rows)} | {tokens - 1})
+    q, k, v = missed(tokens, dim, tokens, rows)
+    cfg = mattn.Config(tokens, 1, 1, dim)
+    out, again = (torch.full((tokens, dim), float("nan"), device="cuda") for _ in range(2))
+    ctx.wide_attention(q, k, v, out, cfg)
+    ctx.wide_attention(q, k, v, again, cfg)
+    torch.cuda.synchronize()
+    assert ctx.wide_attention_route() == 1 and ctx.last_status() == 0
+    assert torch.equal(out, again)
+    scores = q.half().double() @ k.half().double().T / dim ** 0.5
+    want = torch.softmax(scores, -1) @ v.double()
+    # P is rounded to half by 2^-11 of its value, twice where a piece falls below the normal range; V by 2^-11; the weights
+    # that are summed, rounded or not, differ by another 2^-11
+    assert (out - want).abs().max() <= 4 * 2.0 ** -11 * v.abs().max()
+
+
+def test_a_graph_replays_with_and_without_missed_rows(ctx):
+    """One captured call, replayed on operands that the sample misses and on others: the same bytes as calls of their own."""
+    tokens, dim = 2080, 512
+    cfg = mattn.Config(tokens, 1, 1, dim)
+    sets = [missed(tokens, dim, 3, (5, 700, 2079)), make(tokens, dim, 4), missed(tokens, dim, 5, (1, 256))]
+    want = []
+    for x in sets:
+        o = torch.empty((tokens, dim), device="cuda")
+        ctx.wide_attention(*x, o, cfg)
+        want.append((o, ctx.wide_attention_route()))
+    assert [r for _, r in want] == [1, 0, 1]
+    q, k, v = (torch.zeros((tokens, dim), device="cuda") for _ in range(3))
+    out = torch.empty((tokens, dim), device="cuda")
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        ctx.wide_attention(q, k, v, out, cfg)
+    for x, (o, route) in zip(sets, want):
+        for dst, src in zip((q, k, v), x):
+            dst.copy_(src)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, o) and ctx.wide_attention_route() == route
+    assert ctx.last_status() == 0
+
+
+@pytest.mark.parametrize("every", [256, 1])
+def test_missed_rows_do_not_cost_a_second_product(ctx, every):
+    """4096 x 512: one row in 256, or all of them, that the sample misses. Multiplying their blocks again took 1.63 times as
+    long as a call with none; rescaling the rows takes 1.03 and 1.14 times."""
+    tokens, dim = 4096, 512
+    cfg = mattn.Config(tokens, 1, 1, dim)
+    plain = make(tokens, dim, 5)
+    q, k, v = (x.clone() for x in plain)
+    if every == 1:
+        k.copy_(q)  # every query meets itself: 22.6 above the rest
+    else:
+        k[9::every] = q[3::every]  # no key of the sample (every 8th)
+    out = torch.empty_like(q)
+
+    def timed(x):
+        best = []
+        for _ in range(9):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            torch.cuda.synchronize()
+            e0.record()
+            for _ in range(20):
+                ctx.wide_attention(*x, out, cfg)
+            e1.record()
+            torch.cuda.synchronize()
+            best.append(e0.elapsed_time(e1))
+        return min(best)
+
+    timed(plain)
+    base = timed(plain)
+    assert ctx.wide_attention_route() == 0
+    assert timed((q, k, v)) <= 1.3 * base
+    assert ctx.wide_attention_route() == 1

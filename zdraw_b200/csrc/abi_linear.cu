@@ -22,6 +22,8 @@ struct PartSpec {
   float* row_sum = nullptr;          // exp: partial row sums; plain: the rows are divided by their sum
   int n_partial = 0;                 // partial sums per row
   float exp_scale = 0.0f;
+  float* shift = nullptr;            // exp: see LinearPart
+  unsigned int *row_missed = nullptr, *any_missed = nullptr;
   uint32_t n_valid = 0;              // row max / exp: real columns (0 = all n); W then has n_valid rows
 };
 
@@ -31,8 +33,6 @@ struct WideSpec {
   const unsigned int* norms = nullptr;  // row max: see LinearArgs; all of W is n_valid_all rows of k
   uint32_t n_valid_all = 0;
   unsigned int *all_rows = nullptr, *norms_done = nullptr;
-  unsigned int *missed = nullptr, *block_flags = nullptr;  // blocks to be done again (linear.cuh)
-  int run_when = 0;
   bool rows_first = false;        // tile order: across the column blocks of a row block first
   bool early_dependents = false;  // (projections: true)
   int k_splits = 1;               // 2: C holds zeros and each tile's K is walked by two pairs (linear.cuh)
@@ -85,9 +85,6 @@ int run_linear(Ctx* cx, void* stream, const void* a, int n_parts, const PartSpec
   la.n_all = (la.n_valid_all + 255) / 256 * 256;
   la.all_rows = wide.all_rows;
   la.norms_done = wide.norms_done;
-  la.missed = wide.missed;
-  la.block_flags = wide.block_flags;
-  la.run_when = wide.run_when;
   la.rows_first = wide.rows_first ? 1 : 0;
   la.k_splits = wide.k_splits;
   la.early_dependents = wide.early_dependents ? 1 : 0;
@@ -121,6 +118,9 @@ int run_linear(Ctx* cx, void* stream, const void* a, int n_parts, const PartSpec
       lp.row_sum = parts[i].row_sum;
       lp.n_partial = parts[i].n_partial;
       lp.exp_scale = parts[i].exp_scale;
+      lp.shift = parts[i].shift;
+      lp.row_missed = parts[i].row_missed;
+      lp.any_missed = parts[i].any_missed;
       lp.n_valid = static_cast<int>(parts[i].n_valid ? parts[i].n_valid : p->n);
     }
   }
@@ -204,15 +204,16 @@ int zdraw_cuda_wide_attention(void* ctx, void* stream, const float* q, const flo
   // is stored as zeros and skipped by the row maximum).
   const size_t n_pad = (tokens + 255) / 256 * 256;
   const size_t n_partial = n_pad / 128;  // partial row sums: one per 128 columns
-  const size_t n_blocks = (tokens + 255) / 256;
-  const size_t aux_bytes = 4 * (tokens * n_partial + tokens + n_blocks);  // partial sums, row keys, flags of 256 rows
+  const size_t aux_bytes = 4 * (2 * tokens * n_partial + 2 * tokens);  // partial sums, offsets, row keys, row flags
   int rc;
   if ((rc = ensure(cx, cx->wa_q16, n * 2)) || (rc = ensure(cx, cx->wa_k16, n * 2)) || (rc = ensure(cx, cx->wa_vt16, n * 2)) ||
       (rc = ensure(cx, cx->wa_aux, aux_bytes)) || (rc = ensure(cx, cx->wa_p, tokens * n_pad * 2)))
     return rc;
   float* row_sum = static_cast<float*>(cx->wa_aux.p);
-  unsigned int* row_key = reinterpret_cast<unsigned int*>(row_sum + tokens * n_partial);
-  unsigned int* block_flags = row_key + tokens;
+  float* shift = row_sum + tokens * n_partial;
+  unsigned int* row_key = reinterpret_cast<unsigned int*>(shift + tokens * n_partial);
+  unsigned int* row_missed = row_key + tokens;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
   zdraw::WideCast cast = {};
   cast.q = q;
   cast.k = k;
@@ -223,7 +224,7 @@ int zdraw_cuda_wide_attention(void* ctx, void* stream, const float* q, const flo
   cast.tokens = static_cast<int>(tokens);
   cast.ch = static_cast<int>(head_dim);
   cast.row_key = row_key;
-  cast.block_flags = block_flags;
+  cast.row_missed = row_missed;
   cast.state = cx->wa_state;
   // O = P V has few tiles (tokens / 256 x head_dim / 256): where a second half-length round of work items
   // fits the chip better, K is split and the halves are added to an O that the cast launch has zeroed.
@@ -234,23 +235,21 @@ int zdraw_cuda_wide_attention(void* ctx, void* stream, const float* q, const flo
                      zdraw::linear_split_pays(zdraw::linear_tiles(static_cast<int>(tokens), static_cast<int>(head_dim), 1), pairs);
   cast.zero = split ? o : nullptr;
   // kf32_to_h x2, kvt_transpose_h (mvattn_owned.zig:322-330)
-  ZD_CUDA(cx, zdraw::launch_wide_cast(static_cast<cudaStream_t>(stream), cast));
+  ZD_CUDA(cx, zdraw::launch_wide_cast(st, cast));
   cx->wa_ran = true;
   // The scores S = Q K^T (K is already [n][k]) are never stored. One product keeps only row maxima; a
   // second one turns its accumulator into exp(scale (S - max)) in half and keeps partial row sums:
   // recomputing S (k = head_dim is short) costs less than writing and re-reading tokens^2 f32 scores.
   // Softmax does not change when another number than the maximum is subtracted, as long as nothing
   // overflows, so the maxima come from some 512 keys spread over the image (every stride-th one, through
-  // the tensor map's row stride). A row whose largest score lies more than 2^16 above the sample's
-  // (in the exponentials) is noticed by the exp product; its block of 256 rows is then done again from the
-  // exact maxima by two launches that otherwise leave at once. Operands of large norms (scores beyond
-  // kMaxSampledScore possible) get the maxima of all keys from the first launch: nearly every block would be
-  // done again. All of it depends on the data alone. (The
+  // the tensor map's row stride). Where a row's largest score lies 2^16 or more above the sample's (in the
+  // exponentials), the exp product stores the 128 columns concerned under an offset of their own and a
+  // last pass brings such rows to one scale (wide_rescale_kernel). All of it depends on the data alone. (The
   // reference takes the exact f32 maximum of half products, krow_softmax_h, src/metal/mvattn_owned.zig:95-128.)
-  // Together with the split P V and the one cast launch: 94 -> 61 us at 4096 x 512, 759 -> 616 us at 16384 x 512,
-  // against row maxima from e4m3 copies of all keys. A call whose every block is done again multiplies Q by all keys
-  // twice more: 99 us instead of 61 and 1090 instead of 530 (of the same inputs' times after an idle second).
-  // Below 1024 tokens every key is in the sample: its maxima are exact and nothing can need doing again.
+  // A call with a row missed in each block of 256 takes 62.7 us at 4096 x 512 and 537 at 16384 (60.7 and 529 with none;
+  // 99 and 1050 when such blocks were multiplied again under exact maxima), with every row missed 69 and 650 to 735.
+  // Below 1024 tokens every key is in the sample: its maxima are exact and the last pass is left out.
+  // Operands of large norms (scores beyond kMaxSampledScore possible) get the maxima of all keys from the same launch.
   const size_t stride = tokens < 1024 ? 1 : tokens / 512;
   const size_t n_sample = (tokens + stride - 1) / stride;
   zdraw_cuda_linear_params ps = {};
@@ -274,21 +273,26 @@ int zdraw_cuda_wide_attention(void* ctx, void* stream, const float* q, const flo
   ps.n = static_cast<uint32_t>(n_pad);
   ps.ld_w = head_dim;
   part_s.n_valid = static_cast<uint32_t>(tokens);
-  WideSpec when;
-  when.norms_done = cx->wa_state + zdraw::kWideNorms;
-  if (stride > 1) {
-    when.missed = cx->wa_state + zdraw::kWideMissed;
-    when.block_flags = block_flags;
-    when.run_when = zdraw::kRunEstimate;
-  }
   part_s.epilogue = static_cast<uint32_t>(zdraw::kEpilogueExp);
-  if ((rc = run_linear(cx, stream, cx->wa_q16.p, 1, &part_s, nullptr, nullptr, &ps, when)) != 0) return rc;
   if (stride > 1) {
-    when.run_when = zdraw::kRunExact;
-    part_s.epilogue = static_cast<uint32_t>(zdraw::kEpilogueRowMax);
-    if ((rc = run_linear(cx, stream, cx->wa_q16.p, 1, &part_s, nullptr, nullptr, &ps, when)) != 0) return rc;
-    part_s.epilogue = static_cast<uint32_t>(zdraw::kEpilogueExp);
-    if ((rc = run_linear(cx, stream, cx->wa_q16.p, 1, &part_s, nullptr, nullptr, &ps, when)) != 0) return rc;
+    part_s.shift = shift;
+    part_s.row_missed = row_missed;
+    part_s.any_missed = cx->wa_state + zdraw::kWideMissed;
+  }
+  WideSpec exp_spec;
+  exp_spec.norms_done = cx->wa_state + zdraw::kWideNorms;
+  if ((rc = run_linear(cx, stream, cx->wa_q16.p, 1, &part_s, nullptr, nullptr, &ps, exp_spec)) != 0) return rc;
+  if (stride > 1) {
+    zdraw::WideRescale rs = {};
+    rs.p = cx->wa_p.p;
+    rs.ld_p = static_cast<long long>(n_pad);
+    rs.tokens = static_cast<int>(tokens);
+    rs.n_partial = static_cast<int>(n_partial);
+    rs.row_sum = row_sum;
+    rs.shift = shift;
+    rs.row_missed = row_missed;
+    rs.any_missed = cx->wa_state + zdraw::kWideMissed;
+    ZD_CUDA(cx, zdraw::launch_wide_rescale(st, rs, cx->sm_count));
   }
   // O[tokens, head_dim] = (P (V^T)^T) / row sum, f32 out
   zdraw_cuda_linear_params po = {};

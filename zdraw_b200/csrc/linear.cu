@@ -100,11 +100,6 @@ __device__ __forceinline__ uint32_t pack_clamped(float lo, float hi) {
 __global__ void __launch_bounds__(kThreads, 1)
 linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  if (a.run_when == kRunExact) {
-    // A launch of the wide attention that may have nothing to do leaves before it sets anything up.
-    grid_dependency_wait();
-    if (ld_volatile_u32(a.missed) == 0u) return;
-  }
   const uint32_t base = smem_u32(smem_raw);
   volatile uint32_t* flags = reinterpret_cast<volatile uint32_t*>(smem_raw + kOffFlags);
   volatile uint32_t* abort_flag = flags;
@@ -168,10 +163,6 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
   // With k_splits == 2 a tile of C is computed twice, by neighbouring work items that each walk half of K
   // and add their share to C.
   const int n_items = tiles_m * tiles_n * a.n_parts * a.k_splits;
-  // When only some row blocks are to be done again, the others' tiles are passed over by every role alike.
-  const unsigned int* const block_flags =
-      a.run_when == kRunExact ? a.block_flags : nullptr;
-  auto passed_over = [&](int tile_m) -> bool { return block_flags != nullptr && ld_volatile_u32(block_flags + tile_m) == 0u; };
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -189,7 +180,6 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
         const int n_cols = tiles_n * a.n_parts;
         const int col = a.rows_first ? tile % n_cols : tile / tiles_m;
         const int tile_m = a.rows_first ? tile / n_cols : tile % tiles_m;
-        if (passed_over(tile_m)) continue;
         const int tile_n = col % tiles_n;
         const CUtensorMap* tm_w = &maps.w[all_rows ? 1 : col / tiles_n];
         const int row_a = (2 * tile_m + static_cast<int>(rank)) * kTM;
@@ -219,9 +209,7 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
       uint32_t it = 0;
       int local = 0;
       bool ok = *abort_flag == 0u;
-      for (int item = pair; item < n_items && ok; item += n_pairs) {
-        const int tile = item / a.k_splits;
-        if (passed_over(a.rows_first ? tile / (tiles_n * a.n_parts) : tile % tiles_m)) continue;
+      for (int item = pair; item < n_items && ok; item += n_pairs, ++local) {
         const int b = local & 1;
         const uint32_t use = static_cast<uint32_t>(local >> 1);
         // The epilogue warps must have drained this accumulator (first use passes at once).
@@ -246,7 +234,6 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
         }
         if (!ok) break;
         umma_commit_pair(bar(kBarAccFull + b), 3);  // both CTAs' epilogues may read their rows
-        ++local;
       }
       if (!ok) {
         umma_commit_pair(bar(kBarDrain), 1);
@@ -262,16 +249,13 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
     const int quarter = warp & 3;
     const int row = quarter * 32 + lane;
     const uint32_t lane_off = static_cast<uint32_t>(quarter * 32) << 16;
-    int next_local = 0;
+    int local = 0;
     bool ok = __all_sync(0xffffffffu, *abort_flag == 0u);  // warp-uniform
-    for (int item = pair; item < n_items && ok; item += n_pairs) {
+    for (int item = pair; item < n_items && ok; item += n_pairs, ++local) {
       const int tile = item / a.k_splits;
       const int n_cols = tiles_n * a.n_parts;
       const int col = a.rows_first ? tile % n_cols : tile / tiles_m;
-      const int pair_m = a.rows_first ? tile / n_cols : tile % tiles_m;  // block of 256 rows
-      if (passed_over(pair_m)) continue;
-      const int local = next_local++;
-      const int tile_m = 2 * pair_m + static_cast<int>(rank);
+      const int tile_m = 2 * (a.rows_first ? tile / n_cols : tile % tiles_m) + static_cast<int>(rank);
       const int tile_n = col % tiles_n;
       const int half_n = 2 * tile_n + hh;  // this warpgroup's block of 128 columns
       const LinearPart& part = a.part[col / tiles_n];
@@ -335,7 +319,8 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
         // plain: factor of this row; exp: x -> exp2(x * c + bias), bias = -max * c
         float mul = row_factor, bias = 0.0f;
         uint64_t psum = 0ull;  // exp: sums of the even and of the odd columns (+0.0f, +0.0f)
-        float top = -INFINITY;  // exp: largest raw score of the columns that exist
+        float top = -INFINITY;  // exp: largest raw score of this row's 128 columns (of those that exist)
+        float d = 0.0f;         // exp: they are stored times 2^-d
         if (exp_mode) {
           mul = part.exp_scale;
           bias = live ? -key_float(part.row_key[m]) * part.exp_scale : 0.0f;
@@ -382,9 +367,6 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
             const int side = pc & 1;
             uint32_t h[16];
             if (exp_mode) {
-              // (the subtracted maximum may be that of a sample of the keys: the largest raw score is
-              // tracked, one instruction per pair, and the conversion saturates at the largest finite
-              // half, so a row that the sample missed is noticed below and done again)
               const int n_live = part.n_valid - (col_base + 32 * pc);  // columns of this piece that exist
               if (n_live >= 32) {
 #pragma unroll
@@ -430,12 +412,66 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
           tmem_ld_x32(t_acc + 96u, xb);
           piece(2, xa);
           tmem_wait_ld();
-          // The accumulator is in registers: the MMAs of the tile after next may have it now.
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) mbar_arrive_cluster(cluster_map(bar(kBarAccEmpty + b), 0));
-          released = true;
+          // The accumulator is in registers: the MMAs of the tile after next may have it now (unless it may have to
+          // be read again).
+          auto hand_back = [&]() {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(cluster_map(bar(kBarAccEmpty + b), 0));
+            released = true;
+          };
+          if (!exp_mode) hand_back();
           piece(3, xb);
+          if (exp_mode) {
+            // The subtracted maximum may be that of a sample of the keys. Where it is short by 2^16 or more, a row's
+            // 128 columns take an offset of their own, the power of two that brings their largest exponential to
+            // (0.5, 1]: the warp reads its accumulators a second time and converts them with it, and
+            // wide_rescale_kernel brings the row's pieces to one scale. (The exponent is 16 where the half range
+            // ends; a NaN or infinite one counts as well.)
+            const float e_top = fmaf(top, mul, bias);
+            const bool short_max = live && top > -INFINITY && !(e_top < 15.99f);
+            if (__any_sync(0xffffffffu, short_max)) {
+              const bool missed = short_max && part.shift != nullptr;
+              if (missed) d = ceilf(e_top);
+              // bias - d with what its rounding loses (two-sum), so that large scores cost no accuracy
+              const float b_d = bias - d;
+              const float back = b_d - bias;
+              const float lost = (bias - (b_d - back)) - (d + back);
+              // (at 2^26 and more the exponents themselves are off by whole units)
+              if (short_max && !(fmaf(top, mul, b_d) + lost < 15.99f)) atomicOr(a.status, kStExpClamp);
+              psum = 0ull;
+#pragma unroll 1
+              for (int pc = 0; pc < 4; ++pc) {
+                tmem_ld_x32(t_acc + 32u * pc, xa);
+                tmem_wait_ld();
+                const int n_live = part.n_valid - (col_base + 32 * pc);
+                uint4* st = stage + (pc >> 1) * 256;
+                uint32_t h[16];
+#pragma unroll
+                for (int i = 0; i < 16; ++i) {
+                  float e0 = ex2_approx(fmaf(__uint_as_float(xa[2 * i]), mul, b_d) + lost);
+                  float e1 = ex2_approx(fmaf(__uint_as_float(xa[2 * i + 1]), mul, b_d) + lost);
+                  if (2 * i >= n_live) e0 = 0.0f;
+                  if (2 * i + 1 >= n_live) e1 = 0.0f;
+                  h[i] = pack_f16x2_sat(e0, e1);
+                  if (missed) {
+                    // The rounded values: a row that the sample misses is peaked, and what rounding does to its one
+                    // or two large weights then cancels against their sum. (Under the exact maximum the largest
+                    // is 1 and not rounded at all.)
+                    const float2 r = __half22float2(*reinterpret_cast<const __half2*>(h + i));
+                    e0 = r.x;
+                    e1 = r.y;
+                  }
+                  psum = f2_add(psum, f2_pack(e0, e1));
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                  st[lane * 8 + ((4 * (pc & 1) + i) ^ (lane & 7))] =
+                      make_uint4(h[4 * i], h[4 * i + 1], h[4 * i + 2], h[4 * i + 3]);
+              }
+            }
+            hand_back();
+          }
           fence_proxy_async_smem();  // this thread's writes, for the TMA engine
           __syncwarp();
           if (lane == 0 && row0 < a.m) {
@@ -447,15 +483,12 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
         if (exp_mode && live) {
           float even, odd;
           f2_unpack(psum, even, odd);
-          part.row_sum[m * part.n_partial + half_n] = even + odd;
-          // exp2 argument of the largest score: 16 is where the half range ends (NaN also reports).
-          if (top > -INFINITY && !(fmaf(top, mul, bias) < 15.99f)) {
-            if (a.run_when == kRunEstimate) {  // a key outside the sample lies more than 2^16 above it
-              a.block_flags[pair_m] = 1u;
-              *a.missed = 1u;
-            } else {
-              atomicOr(a.status, kStExpClamp);
-            }
+          const long long at = m * part.n_partial + half_n;
+          part.row_sum[at] = d != 0.0f ? -(even + odd) : even + odd;
+          if (d != 0.0f) {
+            part.shift[at] = d;
+            part.row_missed[m] = 1u;
+            *part.any_missed = 1u;
           }
         }
       } else {

@@ -12,17 +12,30 @@ namespace zdraw {
 constexpr int kWideNorms = 0, kWideAllKeys = 2, kWideMissed = 3, kWideStateWords = 4;
 
 // The operands of one call: [tokens][ch] f32 -> q16, k16 [tokens][ch] and vt16 [ch][tokens] in half (clamped);
-// row_key[tokens] and block_flags[ceil(tokens / 256)] zeroed; the norms of state raised to this call's, its other words zeroed.
+// row_key[tokens] and row_missed[tokens] zeroed; the norms of state raised to this call's, its other words zeroed.
 // tokens and ch are multiples of 32.
 struct WideCast {
   const float *q, *k, *v;
   void *q16, *k16, *vt16;
   int tokens, ch;
   unsigned int* row_key;
-  unsigned int* block_flags;
+  unsigned int* row_missed;
   unsigned int* state;
   float* zero;  // optional: [tokens][ch] set to zero
 };
 cudaError_t launch_wide_cast(cudaStream_t stream, const WideCast& args);
+
+// exp(scores) p [tokens][ld_p] in half, n_partial * 128 columns, with the partial sums, offsets and flags that the exp
+// epilogue leaves (LinearPart): rows that are flagged are brought to one scale. Leaves at once when *any_missed is 0.
+struct WideRescale {
+  void* p;
+  long long ld_p;
+  int tokens, n_partial;
+  float* row_sum;
+  const float* shift;
+  const unsigned int* row_missed;
+  const unsigned int* any_missed;
+};
+cudaError_t launch_wide_rescale(cudaStream_t stream, const WideRescale& args, int sm_count);
 
 }  // namespace zdraw

@@ -281,7 +281,7 @@ class Context:
 
     def wide_attention_route(self, stream=None) -> int:
         """How the last ``wide_attention`` call took its row maxima: 0 = from a sample of the keys, 1 = from all keys,
-        for every row (operands of large norms) or for the blocks of 256 rows where the sample had missed it."""
+        for every row (operands of large norms) or for the rows where the sample had missed it."""
         r = C.c_uint32(0)
         self._check(self._lib.zdraw_cuda_wide_attention_route(self._h, self._stream_ptr(stream), C.byref(r)))
         return int(r.value)
