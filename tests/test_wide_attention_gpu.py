@@ -164,7 +164,7 @@ def test_keys_outside_the_sample_are_noticed(ctx, oracle, tokens):
     torch.cuda.synchronize()
     assert ctx.wide_attention_route() == 1 and ctx.last_status() == 0
     assert torch.equal(out, again)
-    assert (out - in_place).abs().max() <= 1e-5  # f32 sums of the two halves of the keys, in one pass or two
+    assert torch.equal(out, in_place)
     got = out.cpu().numpy()
     qh, kh, vh = q.cpu().numpy(), k.cpu().numpy(), v.cpu().numpy()
     for r in (0, 255, 256, 301, 511, 512, tokens - 1):
@@ -303,3 +303,19 @@ def test_missed_rows_do_not_cost_a_second_product(ctx, every):
     assert ctx.wide_attention_route() == 0
     assert timed((q, k, v)) <= 1.3 * base
     assert ctx.wide_attention_route() == 1
+
+
+@pytest.mark.parametrize("tokens,dim", [(32, 32), (320, 512), (2080, 512), (4096, 512)])
+def test_result_in_an_operands_place(ctx, tokens, dim):
+    """The same bytes wherever the result goes: in the place of q, k or v, or overlapping two of them, also where P V is
+    split over the keys (tiles of 256 x 256 that leave half of the pairs of SMs without one)."""
+    x = torch.stack(make(tokens, dim, tokens))
+    cfg = mattn.Config(tokens, 1, 1, dim)
+    want = torch.empty((tokens, dim), device="cuda")
+    ctx.wide_attention(x[0], x[1], x[2], want, cfg)
+    for at in (0, tokens // 2, tokens, 2 * tokens):  # rows of the stacked q, k, v
+        y = x.clone()
+        out = y.view(3 * tokens, dim)[at:at + tokens]
+        ctx.wide_attention(y[0], y[1], y[2], out, cfg)
+        assert torch.equal(out, want)
+    assert ctx.last_status() == 0

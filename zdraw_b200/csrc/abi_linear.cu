@@ -33,6 +33,8 @@ struct WideSpec {
   const unsigned int* norms = nullptr;  // row max: see LinearArgs; all of W is n_valid_all rows of k
   uint32_t n_valid_all = 0;
   unsigned int *all_rows = nullptr, *norms_done = nullptr;
+  float* zero = nullptr;  // zero_n floats set to zero beside the product
+  size_t zero_n = 0;
   bool rows_first = false;        // tile order: across the column blocks of a row block first
   bool early_dependents = false;  // (projections: true)
   int k_splits = 1;               // 2: C holds zeros and each tile's K is walked by two pairs (linear.cuh)
@@ -85,6 +87,8 @@ int run_linear(Ctx* cx, void* stream, const void* a, int n_parts, const PartSpec
   la.n_all = (la.n_valid_all + 255) / 256 * 256;
   la.all_rows = wide.all_rows;
   la.norms_done = wide.norms_done;
+  la.zero = reinterpret_cast<float4*>(wide.zero);
+  la.zero_n4 = static_cast<long long>(wide.zero_n / 4);
   la.rows_first = wide.rows_first ? 1 : 0;
   la.k_splits = wide.k_splits;
   la.early_dependents = wide.early_dependents ? 1 : 0;
@@ -227,13 +231,12 @@ int zdraw_cuda_wide_attention(void* ctx, void* stream, const float* q, const flo
   cast.row_missed = row_missed;
   cast.state = cx->wa_state;
   // O = P V has few tiles (tokens / 256 x head_dim / 256): where a second half-length round of work items
-  // fits the chip better, K is split and the halves are added to an O that the cast launch has zeroed.
+  // fits the chip better, K is split and the halves are added to an O that idle warps of the two launches before have
+  // zeroed. By then the operands have been read, so that the result is the same with O in the place of one of them.
+  // (Zeroed by the cast launch, with P V in one piece for such an O: 60.3 us at 4096 x 512, 66.9 in place; now 59.)
   int pairs = 0;
   ZD_CUDA(cx, zdraw::linear_pairs(cx->sm_count, &pairs));
-  auto overlaps_o = [&](const float* x) { return x < o + n && o < x + n; };
-  const bool split = !overlaps_o(q) && !overlaps_o(k) && !overlaps_o(v) &&  // (an o in an operand's place is zeroed too early)
-                     zdraw::linear_split_pays(zdraw::linear_tiles(static_cast<int>(tokens), static_cast<int>(head_dim), 1), pairs);
-  cast.zero = split ? o : nullptr;
+  const bool split = zdraw::linear_split_pays(zdraw::linear_tiles(static_cast<int>(tokens), static_cast<int>(head_dim), 1), pairs);
   // kf32_to_h x2, kvt_transpose_h (mvattn_owned.zig:322-330)
   ZD_CUDA(cx, zdraw::launch_wide_cast(st, cast));
   cx->wa_ran = true;
@@ -269,6 +272,8 @@ int zdraw_cuda_wide_attention(void* ctx, void* stream, const float* q, const flo
   max_spec.norms = cx->wa_state + zdraw::kWideNorms;
   max_spec.n_valid_all = static_cast<uint32_t>(tokens);
   max_spec.all_rows = cx->wa_state + zdraw::kWideAllKeys;
+  max_spec.zero = split ? o : nullptr;
+  max_spec.zero_n = n / 2;
   if ((rc = run_linear(cx, stream, cx->wa_q16.p, 1, &part_s, nullptr, nullptr, &ps, max_spec)) != 0) return rc;
   ps.n = static_cast<uint32_t>(n_pad);
   ps.ld_w = head_dim;
@@ -281,6 +286,8 @@ int zdraw_cuda_wide_attention(void* ctx, void* stream, const float* q, const flo
   }
   WideSpec exp_spec;
   exp_spec.norms_done = cx->wa_state + zdraw::kWideNorms;
+  exp_spec.zero = split ? o + n / 2 : nullptr;
+  exp_spec.zero_n = n / 2;
   if ((rc = run_linear(cx, stream, cx->wa_q16.p, 1, &part_s, nullptr, nullptr, &ps, exp_spec)) != 0) return rc;
   if (stride > 1) {
     zdraw::WideRescale rs = {};

@@ -243,7 +243,11 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
       }
     }
     __syncwarp();
-  } else if (warp >= 4) {
+  } else if (warp < 4) {
+    if (a.zero != nullptr)
+      for (long long i = 64ll * blockIdx.x + (threadIdx.x - 64); i < a.zero_n4; i += 64ll * gridDim.x)
+        a.zero[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  } else {
     // ------------------------------------------------------------ epilogue (one thread per row and half)
     const int hh = (warp - 4) >> 2;  // which 128 columns of the tile: in the qk epilogue, which of its two heads
     const int quarter = warp & 3;
@@ -656,7 +660,8 @@ cudaError_t launch_linear(cudaStream_t stream, const LinearMaps& maps, const Lin
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute attr[2];
   launch_config(&cfg, attr, stream);
-  cfg.gridDim = dim3(2 * (n_tiles < pairs ? n_tiles : pairs));
+  // (every pair takes part in the zeroing: 2 CTAs would need as long for it as for their tile)
+  cfg.gridDim = dim3(2 * (n_tiles < pairs && args.zero == nullptr ? n_tiles : pairs));
   return cudaLaunchKernelEx(&cfg, linear_kernel, maps, args);
 }
 

@@ -71,6 +71,8 @@ struct LinearArgs {
   int n_all, n_valid_all;
   unsigned int* all_rows;
   unsigned int* norms_done;  // exp: two words that the launch leaves at zero (the norms, for the call after this one)
+  float4* zero;  // optional: zero_n4 pieces set to zero by warps that have no part in the product
+  long long zero_n4;
   int early_dependents;  // 1: the next launch in the stream may be set up before this one ends
   // Tile order: 0 = down the rows of one column block (W stays in L2), 1 = across the column blocks
   // of one row block (A stays in L2).

@@ -50,7 +50,7 @@ __device__ __forceinline__ void transpose_block(const WideCast& a, int block, __
 // Q or K: one warp per row, four floats per lane and step -> four halves (clamped). The block's largest row sum of
 // squares raises *norm as float bits (which order like unsigned integers; a NaN lies above them all), so the
 // result does not depend on the order of the updates.
-__device__ __forceinline__ void cast_block(const WideCast& a, const float* in, __half* out16, int block, bool zero_rows,
+__device__ __forceinline__ void cast_block(const WideCast& a, const float* in, __half* out16, int block,
                                            unsigned int* block_norm, unsigned int* norm) {
   const int row_raw = block * kRowsPerBlock + (static_cast<int>(threadIdx.x) >> 5);
   const bool live = row_raw < a.tokens;
@@ -58,7 +58,6 @@ __device__ __forceinline__ void cast_block(const WideCast& a, const float* in, _
   const int lane = static_cast<int>(threadIdx.x) & 31;
   const float4* src = reinterpret_cast<const float4*>(in + row * a.ch);
   uint2* dst16 = reinterpret_cast<uint2*>(out16 + row * a.ch);
-  float4* zero = zero_rows ? reinterpret_cast<float4*>(a.zero + row * a.ch) : nullptr;
   float ss = 0.0f;
   const int n4 = a.ch / 4;
   // Four loads in flight per lane (512 floats per pass of the warp): the row of the VAE shape in one pass.
@@ -82,7 +81,6 @@ __device__ __forceinline__ void cast_block(const WideCast& a, const float* in, _
       o.x = *reinterpret_cast<const uint32_t*>(&h0);
       o.y = *reinterpret_cast<const uint32_t*>(&h1);
       if (live) dst16[i] = o;
-      if (zero && live) zero[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     }
   }
 #pragma unroll
@@ -106,10 +104,9 @@ __global__ void __launch_bounds__(256) wide_cast_kernel(const WideCast a, int ro
   if (block >= 2 * row_blocks) {
     transpose_block(a, block - 2 * row_blocks, tile);
   } else if (block >= row_blocks) {
-    cast_block(a, a.k, static_cast<__half*>(a.k16), block - row_blocks, false, &block_norm,
-               a.state + kWideNorms + 1);
+    cast_block(a, a.k, static_cast<__half*>(a.k16), block - row_blocks, &block_norm, a.state + kWideNorms + 1);
   } else {
-    cast_block(a, a.q, static_cast<__half*>(a.q16), block, a.zero != nullptr, &block_norm, a.state + kWideNorms);
+    cast_block(a, a.q, static_cast<__half*>(a.q16), block, &block_norm, a.state + kWideNorms);
     const int row = block * kRowsPerBlock + static_cast<int>(threadIdx.x);
     if (threadIdx.x < kRowsPerBlock && row < a.tokens) {
       a.row_key[row] = 0u;  // lies below the key of every float

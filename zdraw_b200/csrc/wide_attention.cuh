@@ -21,7 +21,6 @@ struct WideCast {
   unsigned int* row_key;
   unsigned int* row_missed;
   unsigned int* state;
-  float* zero;  // optional: [tokens][ch] set to zero
 };
 cudaError_t launch_wide_cast(cudaStream_t stream, const WideCast& args);
 
