@@ -16,7 +16,8 @@
  *     reaches the end of the call; the library owns only its context scratch;
  *   - work is enqueued on the caller's stream and the caller synchronises
  *     (as with zdraw_metal_batch_begin/end, metal_api.m:1092-1113);
- *   - a context is used by one host thread at a time;
+ *   - a context is used by one host thread at a time, and its calls share its scratch: calls on several streams
+ *     are ordered by the caller (events), or use a context each;
  *   - struct sizes are asserted on both sides (src/abi_gen.zig:20-57,
  *     src/runtime/abi_assert.zig:25-41): see ZDRAW_CUDA_ATTN_PARAMS_SIZE.
  *
@@ -409,10 +410,9 @@ ZDRAW_CUDA_API int zdraw_cuda_qkv_projection(void *ctx, void *stream, const void
  * half Q, K, V^T; S = Q K^T with f32 accumulation; f32 row softmax with scale 1/sqrt(head_dim)
  * giving half P; O = P V with f32 output), full, non-causal, no mask. q, k, v, o are DEVICE
  * pointers to [tokens][head_dim] f32. tokens (<= 65536) and head_dim (<= 4096) must be multiples
- * of 32, as the reference requires; else the call is declined. o may take the place of q, k or v or overlap them: the
- * result is the same. Scratch (half operands, tokens^2 half exp(scores),
- * row statistics: 0.6 GB at 16384
- * tokens) is grow-only context memory; the f32 scores are never stored.
+ * of 32, as the reference requires; else the call is declined. o may take the place of q, k or v or
+ * overlap them: the result is the same. Scratch (half operands, tokens^2 half exp(scores), row statistics:
+ * 0.6 GB at 16384 tokens) is grow-only context memory; the f32 scores are never stored.
  */
 ZDRAW_CUDA_API int zdraw_cuda_wide_attention(void *ctx, void *stream, const float *q, const float *k, const float *v,
                                              float *o, size_t tokens, size_t head_dim);
@@ -421,10 +421,10 @@ ZDRAW_CUDA_API int zdraw_cuda_wide_attention(void *ctx, void *stream, const floa
  * Which way the last zdraw_cuda_wide_attention call on this context took its row maxima: 0 = from a
  * sample of the keys, for every row (when the operands' norms keep the scores moderate; no row's
  * maximum lay 2^16 or more above its sample in the exponentials), 1 = from all keys, for every row (the
- * reference's exact form) or for the rows where the sample had missed it, which are rescaled. Below 1024 tokens every
- * key is in the sample, and the value only says whether the norms would have called for all keys. The choice is
- * made on the device from the data alone, so repeats take the same route. Plays the part of the bridge's per-route counters (metal_api.m:350, 459). Synchronises
- * `stream`.
+ * reference's exact form) or for the rows where the sample had missed it, which are rescaled. Below
+ * 1024 tokens every key is in the sample, and the value only says whether the norms would have called
+ * for all keys. The choice is made on the device from the data alone, so repeats take the same route.
+ * Plays the part of the bridge's per-route counters (metal_api.m:350, 459). Synchronises `stream`.
  */
 ZDRAW_CUDA_API int zdraw_cuda_wide_attention_route(void *ctx, void *stream, uint32_t *exact_row_max);
 

@@ -1429,7 +1429,7 @@ cudaError_t launch_mask_prepare(cudaStream_t stream, const float* key_mask, long
                                 int tokens, int batch, int* tile_list, long long list_stride) {
   const int n_kv_tiles = (tokens + kBN - 1) / kBN;
   mask_prepare_kernel<<<batch, kMaskThreads, 0, stream>>>(key_mask, mask_batch_stride, tokens, n_kv_tiles, tile_list,
-                                                 list_stride);
+                                                          list_stride);
   return cudaGetLastError();
 }
 

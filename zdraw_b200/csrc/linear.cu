@@ -33,8 +33,6 @@
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
-#include <type_traits>
-
 #include "ptx.cuh"
 
 namespace zdraw {
@@ -149,7 +147,7 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
   const uint32_t tmem_base = flags[1];
   grid_dependency_wait();
   // The kernel behind a projection may set itself up on SMs that run out of work (sub-block at 512 pixels 141.2 us
-  // without, 138.9 with). Not between the wide attention's launches (4096 x 512: 61.7 us without, 62.7 with).
+  // without, 138.9 with). Not between the wide attention's launches (4096 x 512: 61.4 us without, 62.7 with).
   if (a.early_dependents) grid_launch_dependents();
   // Both CTAs of a pair and every role see the same norms: the launch before this one wrote them.
   const bool all_rows = a.norms != nullptr &&

@@ -7,7 +7,7 @@
 
 namespace zdraw {
 
-constexpr int kEpiloguePlain = 0;   // C = A W^T (times row_scale[row] when given)
+constexpr int kEpiloguePlain = 0;   // C = A W^T (rows divided by the sum of row_sum when given)
 constexpr int kEpilogueQk = 1;      // q/k prologue applied to the accumulator
 constexpr int kEpilogueRowMax = 2;  // no C: row_key[row] = max over the row, as an ordered key
 constexpr int kEpilogueExp = 3;     // C = half(exp2((A W^T - max[row]) * exp_scale)), partial row sums
@@ -22,9 +22,9 @@ constexpr int kMaxLinearParts = 3;
 
 // One output of a launch: C_p[m, n] = A[m, k] * W_p[n, k]^T with its own epilogue.
 struct LinearPart {
-  int epilogue;  // kEpiloguePlain | kEpilogueQk
-  int c_f32;     // plain: 1 = f32 C, 0 = f16 C
-  void* c;       // plain: [m][ld_c]; qk: f16 head-major [image][head][token][128]
+  int epilogue;  // kEpilogue*
+  int c_f32;     // plain: 1 = f32 C, 0 = f16 C (exp: f16)
+  void* c;       // plain, exp: [m][ld_c]; qk: f16 head-major [image][head][token][128]
   long long ld_c;
   const float *w_txt, *w_img;  // qk: norm weights [128]
   // row max: out, one ordered key per row (see float_key), zeroed by the caller. exp: in, the same keys;
@@ -48,8 +48,8 @@ struct LinearPart {
 
 // Up to three products that share A (the Q, K and V projections of one activation) run as one
 // launch over n_parts * (n / 256) column blocks. A and every W are reached through tensor maps
-// (f16, 128-byte swizzle, boxes of 64 columns x 128 rows). Tiles are
-// 256 columns x 64 of K; partial tiles read zeros beyond the matrices.
+// (f16, 128-byte swizzle, boxes of 64 columns x 128 rows). Tiles are 256 columns x 64 of K; partial
+// tiles read zeros beyond the matrices.
 struct LinearArgs {
   int m, n, k;
   // 1, or 2 (f32 plain C that holds zeros before the launch, k > 64): each tile's K is walked in two halves by
@@ -81,10 +81,9 @@ struct LinearArgs {
 
 struct LinearMaps {
   CUtensorMap a;
-  CUtensorMap w[kMaxLinearParts];  // unused entries repeat w[0]
-  // Plain parts: C as a 2-D map (columns, rows) with a box of 32 columns x 32 rows, 128-byte
-  // swizzle for f32 and 64-byte swizzle for f16, for the epilogue's tile stores. Unused entries
-  // hold any valid map.
+  CUtensorMap w[kMaxLinearParts];  // unused entries repeat w[0]; with LinearArgs::norms w[1] is all of W
+  // Plain and exp parts: C as a 2-D map (columns, rows) with a box of 128 bytes (32 columns of f32, 64 of
+  // f16) x 32 rows and 128-byte swizzle, for the epilogue's tile stores. Unused entries hold any valid map.
   CUtensorMap c[kMaxLinearParts];
 };
 
