@@ -249,8 +249,8 @@ int zdraw_cuda_wide_attention(void* ctx, void* stream, const float* q, const flo
   // exponentials), the exp product stores the 128 columns concerned under an offset of their own and a
   // last pass brings such rows to one scale (wide_rescale_kernel). All of it depends on the data alone. (The
   // reference takes the exact f32 maximum of half products, krow_softmax_h, src/metal/mvattn_owned.zig:95-128.)
-  // A call with a row missed in each block of 256 takes 62.7 us at 4096 x 512 and 537 at 16384 (60.7 and 529 with none;
-  // 99 and 1050 when such blocks were multiplied again under exact maxima), with every row missed 69 and 650 to 735.
+  // A call with a row missed in each block of 256 takes 60.2 us at 4096 x 512 and 533 at 16384 (59 and 530 with none;
+  // 99 and 1050 when such blocks were multiplied again under exact maxima), with every row missed 64 and 610 to 710.
   // Below 1024 tokens every key is in the sample: its maxima are exact and the last pass is left out.
   // Operands of large norms (scores beyond kMaxSampledScore possible) get the maxima of all keys from the same launch.
   const size_t stride = tokens < 1024 ? 1 : tokens / 512;

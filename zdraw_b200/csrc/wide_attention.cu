@@ -93,7 +93,7 @@ __device__ __forceinline__ void cast_block(const WideCast& a, const float* in, _
 }
 
 // One launch for the three operands (three launches, two memsets and a one-thread kernel took about 25 us of a
-// call at 4096 x 512, this takes 8). Memory-bound: 6 bytes per element, 26 us at 16384 x 512.
+// call at 4096 x 512, this takes 8). Memory-bound: 6 bytes per element, 23 us at 16384 x 512.
 __global__ void __launch_bounds__(256) wide_cast_kernel(const WideCast a, int row_blocks) {
   __shared__ __half tile[kVTile][kVTile + 2];
   __shared__ unsigned int block_norm;
@@ -119,64 +119,67 @@ __global__ void __launch_bounds__(256) wide_cast_kernel(const WideCast a, int ro
 // Brings the rows that the sample of the keys missed to one scale. The exp product has stored each 128 columns of
 // such a row times 2^-d, with a d of their own (0 where the sample served); they become times 2^-D, D the row's
 // largest d, and so do their partial sums. The factors are powers of two: nothing but what falls below the half
-// range is rounded, as it would be under the exact maximum. One block per row and step, 16 bytes per thread.
-// Memory-bound over the rows concerned: a piece whose sum shows that all of it rounds to zero is only written.
+// range is rounded, as it would be under the exact maximum. A piece whose sum shows that all of it rounds to zero
+// is only written.
+// One warp per row and step: a row is a chain of memory latencies (flag, sums, offsets, its elements), so many rows
+// are kept in flight. 16384 x 512 with every row missed: 85 to 164 us (the latter reads and writes all of P, 1.02 GB
+// at 6.2 TB/s); one block per row took 126 to 176, but 18 instead of 21 where 64 rows are missed.
 constexpr int kMaxPartial = 512;  // 65536 tokens
+constexpr int kRescaleWarps = 8;
 __device__ __forceinline__ bool shifted(float sum) { return __float_as_int(sum) < 0 && sum == sum; }
-__global__ void __launch_bounds__(256) wide_rescale_kernel(const WideRescale a) {
-  __shared__ float factor[kMaxPartial];  // of each 128 columns; 0 = all of them round to zero
-  __shared__ float warp_top[8];
+__global__ void __launch_bounds__(32 * kRescaleWarps) wide_rescale_kernel(const WideRescale a) {
+  __shared__ float factors[kRescaleWarps][kMaxPartial];  // of each 128 columns; 0 = all of them round to zero
   grid_dependency_wait();
   if (ld_volatile_u32(a.any_missed) == 0u) return;
   const int warp = static_cast<int>(threadIdx.x) >> 5, lane = static_cast<int>(threadIdx.x) & 31;
-  const int rows_per_pass = 32 * static_cast<int>(gridDim.x);
-  // Every warp reads the flags of the block's next 32 rows at once (17 us instead of 20 where 64 of 16384 are missed).
-  for (int row0 = static_cast<int>(blockIdx.x); row0 < a.tokens; row0 += rows_per_pass) {
-    const int flag_row = row0 + lane * static_cast<int>(gridDim.x);
-    unsigned todo = __ballot_sync(0xffffffffu, flag_row < a.tokens && a.row_missed[flag_row] != 0u);
-    for (; todo != 0u; todo &= todo - 1u) {
-      const int row = row0 + (__ffs(static_cast<int>(todo)) - 1) * static_cast<int>(gridDim.x);
-      float* sums = a.row_sum + static_cast<long long>(row) * a.n_partial;
-      const float* shifts = a.shift + static_cast<long long>(row) * a.n_partial;
-      float top = 0.0f;
-      for (int t = static_cast<int>(threadIdx.x); t < a.n_partial; t += 256)
-        if (shifted(sums[t])) top = fmaxf(top, shifts[t]);
+  float* factor = factors[warp];
+  // From the last row to the first: what is rescaled last is still in L2 when P V begins with the first rows.
+  const int n_warps = kRescaleWarps * static_cast<int>(gridDim.x);
+  for (int back = kRescaleWarps * static_cast<int>(blockIdx.x) + warp; back < a.tokens; back += n_warps) {
+    const int row = a.tokens - 1 - back;
+    if (a.row_missed[row] == 0u) continue;
+    float* sums = a.row_sum + static_cast<long long>(row) * a.n_partial;
+    const float* shifts = a.shift + static_cast<long long>(row) * a.n_partial;
+    float top = 0.0f;
+    for (int t = lane; t < a.n_partial; t += 32)
+      if (shifted(sums[t])) top = fmaxf(top, shifts[t]);
 #pragma unroll
-      for (int off = 16; off > 0; off >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
-      if (lane == 0) warp_top[warp] = top;
-      __syncthreads();
-#pragma unroll
-      for (int w = 0; w < 8; ++w) top = fmaxf(top, warp_top[w]);
-      for (int t = static_cast<int>(threadIdx.x); t < a.n_partial; t += 256) {
-        const float sum = sums[t];
-        const float d = shifted(sum) ? shifts[t] : 0.0f;
-        const int e = static_cast<int>(fmaxf(d - top, -200.0f));
-        const float f = e < -126 ? 0.0f : __uint_as_float(static_cast<uint32_t>(127 + e) << 23);  // 2^e
-        const float scaled = fabsf(sum) * f;  // no element is larger: at 2^-25 and below all of them round to zero
-        sums[t] = scaled;
-        factor[t] = scaled <= 0x1p-25f ? 0.0f : (scaled == scaled ? f : 1.0f);  // NaN stays
-      }
-      __syncthreads();
-      uint4* p = reinterpret_cast<uint4*>(static_cast<__half*>(a.p) + static_cast<long long>(row) * a.ld_p);
-      const int n8 = a.n_partial * 16;  // 8 halves each
-#pragma unroll 4
-      for (int i = static_cast<int>(threadIdx.x); i < n8; i += 256) {
-        const float f = factor[i >> 4];
-        if (f == 1.0f) continue;
-        uint4 x = make_uint4(0u, 0u, 0u, 0u);
-        if (f != 0.0f) {
-          x = p[i];
-          uint32_t* h = reinterpret_cast<uint32_t*>(&x);
-#pragma unroll
-          for (int j = 0; j < 4; ++j) {
-            const float2 v = __half22float2(*reinterpret_cast<const __half2*>(h + j));
-            h[j] = pack_f16x2(v.x * f, v.y * f);
-          }
-        }
-        p[i] = x;
-      }
-      __syncthreads();  // factor and warp_top are used again
+    for (int off = 16; off > 0; off >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
+    for (int t = lane; t < a.n_partial; t += 32) {
+      const float sum = sums[t];
+      const float d = shifted(sum) ? shifts[t] : 0.0f;
+      const int e = static_cast<int>(fmaxf(d - top, -200.0f));
+      const float f = e < -126 ? 0.0f : __uint_as_float(static_cast<uint32_t>(127 + e) << 23);  // 2^e
+      const float scaled = fabsf(sum) * f;  // no element is larger: at 2^-25 and below all of them round to zero
+      sums[t] = scaled;
+      factor[t] = scaled <= 0x1p-25f ? 0.0f : (scaled == scaled ? f : 1.0f);  // NaN stays
     }
+    __syncwarp();
+    uint4* p = reinterpret_cast<uint4*>(static_cast<__half*>(a.p) + static_cast<long long>(row) * a.ld_p);
+    const int n8 = a.n_partial * 16;  // 8 halves each; a multiple of 32
+    for (int i0 = lane; i0 < n8; i0 += 8 * 32) {
+      uint4 x[8];
+      float f[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int i = i0 + 32 * u;
+        f[u] = i < n8 ? factor[i >> 4] : 1.0f;
+        x[u] = make_uint4(0u, 0u, 0u, 0u);
+        if (f[u] != 0.0f && f[u] != 1.0f) x[u] = p[i];
+      }
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        if (f[u] == 1.0f) continue;
+        uint32_t* h = reinterpret_cast<uint32_t*>(&x[u]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float2 v = __half22float2(*reinterpret_cast<const __half2*>(h + j));
+          h[j] = pack_f16x2(v.x * f[u], v.y * f[u]);
+        }
+        p[i0 + 32 * u] = x[u];
+      }
+    }
+    __syncwarp();  // the factors are used again
   }
 }
 
@@ -200,9 +203,9 @@ cudaError_t launch_wide_cast(cudaStream_t stream, const WideCast& args) {
 cudaError_t launch_wide_rescale(cudaStream_t stream, const WideRescale& args, int sm_count) {
   if (args.n_partial > kMaxPartial) return cudaErrorInvalidValue;
   cudaLaunchConfig_t cfg = {};
-  const int blocks = 8 * sm_count;  // as many as are resident at once
-  cfg.gridDim = dim3(args.tokens < blocks ? args.tokens : blocks);
-  cfg.blockDim = dim3(256);
+  const int blocks = 8 * sm_count, needed = (args.tokens + kRescaleWarps - 1) / kRescaleWarps;
+  cfg.gridDim = dim3(needed < blocks ? needed : blocks);
+  cfg.blockDim = dim3(32 * kRescaleWarps);
   cfg.stream = stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
