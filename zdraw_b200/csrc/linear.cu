@@ -95,6 +95,9 @@ __device__ __forceinline__ uint32_t pack_clamped(float lo, float hi) {
   return *reinterpret_cast<const uint32_t*>(&h);
 }
 
+// kSampled: the wide attention's row-max launch, which chooses its W by the operands' norms. A kernel of its own: with
+// the choice in all of them the other launches were 0.3 to 0.5 us longer without ever taking it (16 and 33 us).
+template <bool kSampled>
 __global__ void __launch_bounds__(kThreads, 1)
 linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -107,7 +110,11 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_cta_rank();  // 0: issues the pair's MMAs
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
+  int tiles_n = (a.n + kTN - 1) / kTN;                  // column blocks of one part (the last may be partial)
   const int tiles_m = (a.m + 2 * kTM - 1) / (2 * kTM);  // pair tiles: 256 rows
+  // With k_splits == 2 a tile of C is computed twice, by neighbouring work items that each walk half of K
+  // and add their share to C.
+  int n_items = tiles_m * tiles_n * a.n_parts * a.k_splits;
   // A stage is a 128-byte slice of K per row; rows, columns and K beyond the matrices read as zeros.
   const int k_steps_all = (a.k + kTK - 1) / kTK;
   auto first_k = [&](int item) { return (item % a.k_splits) * (k_steps_all / a.k_splits); };
@@ -149,18 +156,17 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
   // The kernel behind a projection may set itself up on SMs that run out of work (sub-block at 512 pixels 141.2 us
   // without, 138.9 with). Not between the wide attention's launches (4096 x 512: 61.4 us without, 62.7 with).
   if (a.early_dependents) grid_launch_dependents();
-  // Both CTAs of a pair and every role see the same norms: the launch before this one wrote them.
-  const bool all_rows = a.norms != nullptr &&
-                        !(sqrtf(__uint_as_float(ld_volatile_u32(a.norms))) * sqrtf(__uint_as_float(ld_volatile_u32(a.norms + 1))) *
-                              a.norm_scale <= kMaxSampledScore);
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    if (all_rows) *a.all_rows = 1u;
-    if (a.norms_done != nullptr) a.norms_done[0] = a.norms_done[1] = 0u;
+  bool all_rows = false;
+  if constexpr (kSampled) {
+    // Both CTAs of a pair and every role see the same norms: the launch before this one wrote them.
+    const float q2 = __uint_as_float(ld_volatile_u32(a.norms)), k2 = __uint_as_float(ld_volatile_u32(a.norms + 1));
+    all_rows = !(sqrtf(q2) * sqrtf(k2) * a.norm_scale <= kMaxSampledScore);
+    if (all_rows) {
+      tiles_n = (a.n_all + kTN - 1) / kTN;
+      n_items = tiles_m * tiles_n;
+      if (blockIdx.x == 0 && threadIdx.x == 0) *a.all_rows = 1u;
+    }
   }
-  const int tiles_n = ((all_rows ? a.n_all : a.n) + kTN - 1) / kTN;  // column blocks of one part (the last may be partial)
-  // With k_splits == 2 a tile of C is computed twice, by neighbouring work items that each walk half of K
-  // and add their share to C.
-  const int n_items = tiles_m * tiles_n * a.n_parts * a.k_splits;
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -242,6 +248,7 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
     }
     __syncwarp();
   } else if (warp < 4) {
+    if (a.norms_done != nullptr && blockIdx.x == 0 && threadIdx.x == 64) a.norms_done[0] = a.norms_done[1] = 0u;
     if (a.zero != nullptr)
       for (long long i = 64ll * blockIdx.x + (threadIdx.x - 64); i < a.zero_n4; i += 64ll * gridDim.x)
         a.zero[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -608,7 +615,9 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
 }  // namespace
 
 cudaError_t linear_configure() {
-  return cudaFuncSetAttribute(linear_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+  const cudaError_t err = cudaFuncSetAttribute(linear_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
+  if (err != cudaSuccess) return err;
+  return cudaFuncSetAttribute(linear_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
 }
 
 namespace {
@@ -643,7 +652,7 @@ cudaError_t linear_pairs(int sm_count, int* out) {
     cudaLaunchAttribute attr[2];
     launch_config(&cfg, attr, nullptr);
     cfg.gridDim = dim3(2 * (sm_count / 2));
-    err = cudaOccupancyMaxActiveClusters(&pairs, linear_kernel, &cfg);
+    err = cudaOccupancyMaxActiveClusters(&pairs, linear_kernel<false>, &cfg);
     if (err != cudaSuccess) return err;
     if (pairs <= 0) return cudaErrorLaunchOutOfResources;
     if (pairs > sm_count / 2) pairs = sm_count / 2;
@@ -660,7 +669,8 @@ cudaError_t launch_linear(cudaStream_t stream, const LinearMaps& maps, const Lin
   launch_config(&cfg, attr, stream);
   // (every pair takes part in the zeroing: 2 CTAs would need as long for it as for their tile)
   cfg.gridDim = dim3(2 * (n_tiles < pairs && args.zero == nullptr ? n_tiles : pairs));
-  return cudaLaunchKernelEx(&cfg, linear_kernel, maps, args);
+  if (args.norms != nullptr) return cudaLaunchKernelEx(&cfg, linear_kernel<true>, maps, args);
+  return cudaLaunchKernelEx(&cfg, linear_kernel<false>, maps, args);
 }
 
 }  // namespace zdraw
