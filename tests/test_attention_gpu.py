@@ -462,3 +462,23 @@ def test_growing_row_maxima_rescale_path_on_both_kernels(ctx, oracle):
     err = np.abs(small - want)
     assert err.max() <= 2e-2 and err.mean() <= 2e-3, (err.max(), err.mean())
     np.testing.assert_array_equal(small, large[:, :2])
+
+
+@pytest.mark.parametrize("steps", range(1, 10))
+def test_number_of_kv_steps_on_both_kernels(ctx, oracle, steps):
+    """1 to 9 K/V steps: the rings of three and four tiles wrap, the first score products are issued ahead, the last
+    have no successor. Key norms grow from step to step, so that the maxima of some rows move late (rescale of O) and
+    of others do not. The last step is whole, or has one key."""
+    heads = 2
+    for tokens in (128 * steps, 128 * (steps - 1) + 1):
+        rng = np.random.default_rng(100 * steps + tokens)
+        q, k, v = (rng.standard_normal((tokens, heads, 128)).astype(np.float16) for _ in range(3))
+        k = (k * (0.5 + 1.5 * np.arange(tokens)[:, None, None] / tokens)).astype(np.float16)
+        want = oracle.sdpa(q.astype(np.float32), k.astype(np.float32), v.astype(np.float32), heads)
+        got = {}
+        for form in (_lib.KERNEL_TWO_TILE, _lib.KERNEL_ONE_TILE):
+            got[form] = np.full(q.shape, np.nan, np.float16)
+            ctx.run(got[form], q, k, v, mattn.Config(tokens, heads, heads, 128), kernel=form)
+            # Half weights and a half result, each off by at most 2^-11 of |v| <= 5: 5e-3.
+            assert np.abs(got[form].astype(np.float32) - want).max() <= 5e-3, f"{tokens} tokens, form {form}"
+        np.testing.assert_array_equal(got[_lib.KERNEL_TWO_TILE].view(np.uint16), got[_lib.KERNEL_ONE_TILE].view(np.uint16))

@@ -30,11 +30,12 @@
 // still being reduced (the reduction is off the chain S -> P -> P V -> next S).
 //
 // P reaches the MMA warp in three pieces (keys [0,64), [64,96), [96,128)), so that O += P V
-// starts while the last keys are still being exponentiated. The MMA-issuing thread probes the
+// starts while the last keys are still being exponentiated. The MMA-issuing warp probes the
 // barrier of the next piece (or of the next K/V slot) inside the asm block that issues the
 // current batch of MMAs: a ready-barrier poll costs 100-170 clocks, which would otherwise be
 // tensor-pipe idle time after every batch (measured: five exposed polls per K/V step take the
-// issuing thread from 2048 to 2890 clocks per step, probes inside the batches to 2200).
+// issuing thread from 2048 to 2890 clocks per step, probes inside the batches to 2200). The whole
+// warp runs the issuing loop, converged, and an elected lane issues (see umma_ts_warp).
 //
 // TMEM columns: [0,128) S/P tile 0, [128,256) S/P tile 1, [256,384) O tile 0,
 // [384,512) O tile 1. P (fp16) overwrites the first 64 columns of its S.
@@ -111,6 +112,12 @@ __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile
   return mbar_wait_bounded(bar, parity, abort_flag, status, code, kWaitLimitNs);
 }
 
+// The same for a whole converged warp.
+__device__ __forceinline__ bool wait_bar_warp(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag,
+                                              uint32_t* status, uint32_t code) {
+  return __all_sync(0xffffffffu, wait_bar(bar, parity, abort_flag, status, code));
+}
+
 // 2^x for a packed pair on the FMA pipe. x is clamped to >= -126 so the exponent arithmetic
 // cannot wrap; x <= 8 + small by construction (lazy rescale threshold). Relative error of the
 // cubic on [-0.5, 0.5] is 7.5e-5, below the fp16 rounding of P (4.9e-4).
@@ -171,11 +178,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   volatile uint32_t* abort_flag = flags;
   auto bar = [&](int i) -> uint32_t { return base + kOffBar + 8u * static_cast<uint32_t>(i); };
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);  // known to be the same in the warp
   const int lane = threadIdx.x & 31;
   const bool tracing = kTrace && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0;
   auto stamp = [&](int role, int step, int event) {
-    if (kTrace && tracing && step < kTraceIters)
+    if (kTrace && tracing && lane == 0 && step < kTraceIters)
       a.trace[(role * kTraceIters + step) * kTraceEvents + event] = static_cast<unsigned long long>(clock64());
   };
   const int q_tile0 = blockIdx.x * 2;
@@ -211,7 +218,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = flags[1];
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, flags[1], 0);
 
   // Everything above overlaps the tail of the preceding kernel (the prologue) when the launch
   // allows it; from here on this kernel reads what earlier kernels wrote.
@@ -228,7 +235,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 
   // Active K/V tiles of this image: all of them, or the list a key mask left.
   const int* tile_list = a.tile_list ? a.tile_list + static_cast<size_t>(img) * a.tile_list_stride : nullptr;
-  const int n_act = tile_list ? tile_list[0] : a.n_kv_tiles;
+  const int n_act = __shfl_sync(0xffffffffu, tile_list ? tile_list[0] : a.n_kv_tiles, 0);
   auto tile_entry = [&](int jj) -> int { return tile_list ? tile_list[1 + jj] : jj; };
 
   if (warp < 4) {
@@ -283,7 +290,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
       __syncwarp();
     } else if (warp == 1) {
       // ---------------------------------------------------------- MMA issuer
-      if (lane == 0 && n_act > 0) {
+      if (n_act > 0) {
         constexpr uint32_t idesc_qk = umma_idesc_f16(kBM, kBN, 0, 0);
         constexpr uint32_t idesc_pv = umma_idesc_f16(kBM, 128, 0, 1);
 
@@ -296,7 +303,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
 #pragma unroll
           for (int k = 0; k < 8; ++k) {
             const uint32_t off = static_cast<uint32_t>((k >> 2) * kHalfBytes + (k & 3) * 32) >> 4;
-            umma_ss(d_tmem, desc_q + off, desc_k + off, idesc_qk, k > 0 ? 1u : 0u);
+            umma_ss_warp(d_tmem, desc_q + off, desc_k + off, idesc_qk, k > 0 ? 1u : 0u);
           }
         };
         // O_t (+)= P_t V: the K dimension is 128 keys = 8 steps of 16 keys (2048 bytes of V
@@ -309,22 +316,22 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           const uint32_t d_tmem = tmem_base + 256u + 128u * t;
 #pragma unroll
           for (int k = k0; k < k1; ++k) {
-            umma_ts(d_tmem, p_tmem + 8u * k, desc_v + ((2048u * k) >> 4), idesc_pv,
+            umma_ts_warp(d_tmem, p_tmem + 8u * k, desc_v + ((2048u * k) >> 4), idesc_pv,
                     (accumulate || k > 0) ? 1u : 0u);
           }
         };
 
-        bool ok = wait_bar(bar(kBarQFull + 0), 0, abort_flag, a.status, kStMma) &&
-                  wait_bar(bar(kBarQFull + 1), 0, abort_flag, a.status, kStMma);
-        if (ok) ok = wait_bar(bar(kBarKVFull + 0), 0, abort_flag, a.status, kStMma);
+        bool ok = wait_bar_warp(bar(kBarQFull + 0), 0, abort_flag, a.status, kStMma) &&
+                  wait_bar_warp(bar(kBarQFull + 1), 0, abort_flag, a.status, kStMma);
+        if (ok) ok = wait_bar_warp(bar(kBarKVFull + 0), 0, abort_flag, a.status, kStMma);
         if (ok) {
           tc_fence_after();
           const uint32_t k_addr = base + kOffKV + kTileBytes;  // pair 0: K_0 in the second half of slot 0
           issue_qk(0, k_addr);
-          umma_commit(bar(kBarSFull + 0));
+          umma_commit_warp(bar(kBarSFull + 0));
           issue_qk(1, k_addr);
-          umma_commit(bar(kBarSFull + 1));
-          umma_commit(bar(kBarKVEmpty + 0));
+          umma_commit_warp(bar(kBarSFull + 1));
+          umma_commit_warp(bar(kBarKVEmpty + 0));
         }
         // Steps with a successor: every barrier the next batch of MMAs depends on is probed
         // ahead of the current batch (inside its asm block), so a probe that finds the phase
@@ -337,8 +344,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
           const uint32_t pair = static_cast<uint32_t>(jj0) + 1u;
           const uint32_t slot = pair % kPairStages;
           const uint32_t par = static_cast<uint32_t>(jj0) & 1u;
-          if (!rdy_kv) ok = wait_bar(bar(kBarKVFull + slot), (pair / kPairStages) & 1u, abort_flag, a.status, kStMma);
-          if (ok && !rdy_p) ok = wait_bar(bar(kBarPFull + 0), par, abort_flag, a.status, kStMma);
+          if (!rdy_kv) ok = wait_bar_warp(bar(kBarKVFull + slot), (pair / kPairStages) & 1u, abort_flag, a.status, kStMma);
+          if (ok && !rdy_p) ok = wait_bar_warp(bar(kBarPFull + 0), par, abort_flag, a.status, kStMma);
           if (!ok) break;
           tc_fence_after();
           const uint32_t v_addr = base + kOffKV + slot * 2 * kTileBytes;
@@ -361,7 +368,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 const uint32_t r = (n == 4) ? umma_ts4_probe(d_tmem, pa, dv, idesc_pv, (i == 0) ? acc : 1u, nb, par)
                                             : umma_ts2_probe(d_tmem, pa, dv, idesc_pv, (i == 0) ? acc : 1u, nb, par);
                 if (!r) {
-                  ok = wait_bar(nb, par, abort_flag, a.status, kStMma);
+                  ok = wait_bar_warp(nb, par, abort_flag, a.status, kStMma);
                   if (!ok) break;
                 }
                 tc_fence_after();
@@ -371,9 +378,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 uint32_t r1, r2;
                 if (n == 4) umma_ts4_ss8_probe2(d_tmem, pa, dv, idesc_pv, p_tmem, desc_q, desc_k, idesc_qk, nb, par, nb, par, r1, r2);
                 else umma_ts2_ss8_probe2(d_tmem, pa, dv, idesc_pv, p_tmem, desc_q, desc_k, idesc_qk, nb, par, nb, par, r1, r2);
-                umma_commit(bar(kBarSFull + 0));
+                umma_commit_warp(bar(kBarSFull + 0));
                 if (!r1) {
-                  ok = wait_bar(nb, par, abort_flag, a.status, kStMma);
+                  ok = wait_bar_warp(nb, par, abort_flag, a.status, kStMma);
                   if (!ok) break;
                 }
                 tc_fence_after();
@@ -385,20 +392,20 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
                 else
                   umma_ts2_ss8_probe2(d_tmem, pa, dv, idesc_pv, p_tmem, desc_q, desc_k, idesc_qk, bar(kBarKVFull + nslot),
                                       (npair / kPairStages) & 1u, bar(kBarPFull + 0), par ^ 1u, rdy_kv, rdy_p);
-                umma_commit(bar(kBarSFull + 1));
+                umma_commit_warp(bar(kBarSFull + 1));
               }
             }
             if (!ok) break;
           }
           if (!ok) break;
-          umma_commit(bar(kBarKVEmpty + slot));
+          umma_commit_warp(bar(kBarKVEmpty + slot));
         }
         // The last step (or the only one) takes the plain path below; what was probed for it counts.
         for (int jj = jj0; jj < n_act && ok; ++jj) {
           const uint32_t pair = static_cast<uint32_t>(jj) + 1u;
           const uint32_t slot = pair % kPairStages;
           stamp(4, jj, 0);
-          ok = wait_bar(bar(kBarKVFull + slot), (pair / kPairStages) & 1u, abort_flag, a.status, kStMma);
+          ok = wait_bar_warp(bar(kBarKVFull + slot), (pair / kPairStages) & 1u, abort_flag, a.status, kStMma);
           if (!ok) break;
           stamp(4, jj, 1);
           const bool has_next = (jj + 1 < n_act);
@@ -411,7 +418,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             stamp(0, jj, 4 * t + 0);
 #pragma unroll
             for (int i = 0; i < kPieces; ++i) {
-              ok = wait_bar(bar(kBarPFull + kPieces * t + i), static_cast<uint32_t>(jj) & 1u, abort_flag, a.status, kStMma);
+              ok = wait_bar_warp(bar(kBarPFull + kPieces * t + i), static_cast<uint32_t>(jj) & 1u, abort_flag, a.status, kStMma);
               if (!ok) break;
               tc_fence_after();
               if (i < 2) stamp(0, jj, 4 * t + 1 + i);
@@ -420,20 +427,20 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
             if (!ok) break;
             if (has_next) {
               issue_qk(t, k_addr);
-              umma_commit(bar(kBarSFull + t));
+              umma_commit_warp(bar(kBarSFull + t));
             } else {
-              umma_commit(bar(kBarOFull + t));
+              umma_commit_warp(bar(kBarOFull + t));
             }
             stamp(0, jj, 4 * t + 3);
           }
           if (!ok) break;
-          umma_commit(bar(kBarKVEmpty + slot));
+          umma_commit_warp(bar(kBarKVEmpty + slot));
         }
         if (!ok) {
           // Wait (bounded) for MMAs already issued before TMEM is released.
-          umma_commit(bar(kBarDrain));
+          umma_commit_warp(bar(kBarDrain));
           const uint64_t t0 = globaltimer_ns();
-          while (!mbar_try_wait(bar(kBarDrain), 0) && globaltimer_ns() - t0 < kWaitLimitNs) {
+          while (!__all_sync(0xffffffffu, mbar_try_wait(bar(kBarDrain), 0) || globaltimer_ns() - t0 >= kWaitLimitNs)) {
           }
         }
       }
@@ -767,7 +774,7 @@ attn_fwd_steps_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   volatile float* l_run = m_ref + kBM;
   auto bar = [&](int i) -> uint32_t { return base + kS1OffBar + 8u * static_cast<uint32_t>(i); };
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);  // known to be the same in the warp
   const int lane = threadIdx.x & 31;
   const int q_tile = blockIdx.x;
   const int head = blockIdx.y;
@@ -799,13 +806,13 @@ attn_fwd_steps_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = flags[1];
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, flags[1], 0);
   grid_dependency_wait();
 
   auto c1 = [&](int hm, int tok) { return hm ? tok : head; };
   auto c2 = [&](int hm, int tok) { return hm ? head : tok; };
   const int* tile_list = a.tile_list ? a.tile_list + static_cast<size_t>(img) * a.tile_list_stride : nullptr;
-  const int n_act = tile_list ? tile_list[0] : a.n_kv_tiles;
+  const int n_act = __shfl_sync(0xffffffffu, tile_list ? tile_list[0] : a.n_kv_tiles, 0);
   auto tile_entry = [&](int jj) -> int { return tile_list ? tile_list[1 + jj] : jj; };
 
   if (warp < 4) {
@@ -860,7 +867,7 @@ attn_fwd_steps_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       __syncwarp();
     } else if (warp == 1) {
       // ---------------------------------------------------------- MMA issuer
-      if (lane == 0 && n_act > 0) {
+      if (n_act > 0) {
         constexpr uint32_t idesc_qk = umma_idesc_f16(kBM, kBN, 0, 0);
         constexpr uint32_t idesc_pv = umma_idesc_f16(kBM, 128, 0, 1);
         constexpr uint32_t kHi = kHalfBytes >> 4;  // second 64-column block of a K-major operand (descriptor units)
@@ -876,20 +883,20 @@ attn_fwd_steps_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 #pragma unroll
           for (int k = 0; k < 8; ++k) {
             const uint32_t off = (k >> 2) * kHi + (k & 3) * 2;
-            umma_ss(d_s, desc_q + off, dk + off, idesc_qk, k > 0 ? 1u : 0u);
+            umma_ss_warp(d_s, desc_q + off, dk + off, idesc_qk, k > 0 ? 1u : 0u);
           }
-          umma_commit(bar(kS1BarSFull + i % 3));
-          umma_commit(bar(kS1BarKEmpty + i % 3));
+          umma_commit_warp(bar(kS1BarSFull + i % 3));
+          umma_commit_warp(bar(kS1BarKEmpty + i % 3));
         };
 
-        bool ok = wait_bar(bar(kS1BarQFull), 0, abort_flag, a.status, kStMma);
-        if (ok) ok = wait_bar(bar(kS1BarKFull + 0), 0, abort_flag, a.status, kStMma);
+        bool ok = wait_bar_warp(bar(kS1BarQFull), 0, abort_flag, a.status, kStMma);
+        if (ok) ok = wait_bar_warp(bar(kS1BarKFull + 0), 0, abort_flag, a.status, kStMma);
         if (ok) {
           tc_fence_after();
           issue_qk(0);
         }
         if (ok && n_act > 1) {
-          ok = wait_bar(bar(kS1BarKFull + 1), 0, abort_flag, a.status, kStMma);
+          ok = wait_bar_warp(bar(kS1BarKFull + 1), 0, abort_flag, a.status, kStMma);
           if (ok) {
             tc_fence_after();
             issue_qk(1);
@@ -906,22 +913,22 @@ attn_fwd_steps_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
           if (j + 2 < n_act) {
             const int i = j + 2;
             if (!rdy_k) {
-              ok = wait_bar(bar(kS1BarKFull + i % 3), par3(i), abort_flag, a.status, kStMma);
+              ok = wait_bar_warp(bar(kS1BarKFull + i % 3), par3(i), abort_flag, a.status, kStMma);
               if (!ok) break;
             }
             tc_fence_after();
             const uint64_t dk = desc_k(i);
             umma_ss8_probe2(tmem_base + 128u * (static_cast<uint32_t>(i) % 3u), desc_q, dk, idesc_qk, desc_q + kHi, dk + kHi,
                             bar(kS1BarVFull + b), par, bar(kS1BarPFull + kPieces * b), par, rdy_v, rdy_p);
-            umma_commit(bar(kS1BarSFull + i % 3));
-            umma_commit(bar(kS1BarKEmpty + i % 3));
+            umma_commit_warp(bar(kS1BarSFull + i % 3));
+            umma_commit_warp(bar(kS1BarKEmpty + i % 3));
           }
           if (!rdy_v) {
-            ok = wait_bar(bar(kS1BarVFull + b), par, abort_flag, a.status, kStMma);
+            ok = wait_bar_warp(bar(kS1BarVFull + b), par, abort_flag, a.status, kStMma);
             if (!ok) break;
           }
           if (!rdy_p) {
-            ok = wait_bar(bar(kS1BarPFull + kPieces * b), par, abort_flag, a.status, kStMma);
+            ok = wait_bar_warp(bar(kS1BarPFull + kPieces * b), par, abort_flag, a.status, kStMma);
             if (!ok) break;
           }
           tc_fence_after();
@@ -940,7 +947,7 @@ attn_fwd_steps_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
               // nothing left to probe: plain issue
 #pragma unroll
               for (int k = k0; k < k0 + n; ++k)
-                umma_ts(d_o, p_tmem + 8u * k, dv + 128u * k, idesc_pv, 1u);
+                umma_ts_warp(d_o, p_tmem + 8u * k, dv + 128u * k, idesc_pv, 1u);
               r = 0;
             } else {
               r = (n == 4) ? umma_ts4_probe(d_o, p_tmem + 8u * k0, dv + 128u * k0, idesc_pv, acc, nb, np)
@@ -950,20 +957,20 @@ attn_fwd_steps_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
               rdy_k = probe_k ? r : 0u;
             } else {
               if (!r) {
-                ok = wait_bar(nb, np, abort_flag, a.status, kStMma);
+                ok = wait_bar_warp(nb, np, abort_flag, a.status, kStMma);
                 if (!ok) break;
               }
               tc_fence_after();
             }
           }
           if (!ok) break;
-          umma_commit(bar(kS1BarVEmpty + b));  // V slot free; also: P V of step j is complete
-          if (j + 1 == n_act) umma_commit(bar(kS1BarOFull));
+          umma_commit_warp(bar(kS1BarVEmpty + b));  // V slot free; also: P V of step j is complete
+          if (j + 1 == n_act) umma_commit_warp(bar(kS1BarOFull));
         }
         if (!ok) {
-          umma_commit(bar(kS1BarDrain));
+          umma_commit_warp(bar(kS1BarDrain));
           const uint64_t t0 = globaltimer_ns();
-          while (!mbar_try_wait(bar(kS1BarDrain), 0) && globaltimer_ns() - t0 < kWaitLimitNs) {
+          while (!__all_sync(0xffffffffu, mbar_try_wait(bar(kS1BarDrain), 0) || globaltimer_ns() - t0 >= kWaitLimitNs)) {
           }
         }
       }

@@ -171,6 +171,45 @@ __device__ __forceinline__ void umma_commit(uint32_t bar) {
                : "memory");
 }
 
+// The same from a whole converged warp: one lane is elected, the same one every time. With the issuing role in an
+// `if (lane == 0)` the operands, computed in divergent code, took an MMA about 82 clocks to issue beside eight busy
+// softmax warps, longer than the 64 it executes (M128 N128 K16, whatever else the SM does: operands from shared
+// memory or TMEM, beside TMA writes, tcgen05.ld/st, ex2 and st.shared, each measured); from converged code a batch
+// of eight is issued in 330 to 530 clocks. A K/V step of attn_fwd_kernel went from 3190 to 2830 clocks.
+__device__ __forceinline__ void umma_ts_warp(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                             uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p, pe;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "elect.sync _|pe, 0xffffffff;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t"
+      "}" ::"r"(d_tmem),
+      "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void umma_ss_warp(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                             uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p, pe;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "elect.sync _|pe, 0xffffffff;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+      "}" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit_warp(uint32_t bar) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred pe;\n\t"
+      "elect.sync _|pe, 0xffffffff;\n\t"
+      "@pe tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t"
+      "}" ::"r"(bar)
+      : "memory");
+}
+
 // Batches of MMAs in one asm block with an mbarrier probe issued ahead of them: the probe's
 // result (has the phase `parity` of `bar` completed?) is read only after the MMAs have been
 // issued, so its latency (about a hundred clocks) overlaps their issue instead of leaving the
@@ -181,9 +220,10 @@ __device__ __forceinline__ uint32_t umma_ts4_probe(uint32_t d_tmem, uint32_t a_t
   uint32_t ready;
   asm volatile(
       "{\n\t"
-      ".reg .pred pw, pa, pt;\n\t"
+      ".reg .pred pe, pw, pa, pt;\n\t"
       ".reg .b64 d1, d2, d3;\n\t"
       ".reg .b32 a1, a2, a3;\n\t"
+      "elect.sync _|pe, 0xffffffff;\n\t"
       "mbarrier.test_wait.parity.shared::cta.b64 pw, [%6], %7;\n\t"
       "setp.ne.b32 pa, %5, 0;\n\t"
       "setp.eq.b32 pt, 0, 0;\n\t"
@@ -193,10 +233,11 @@ __device__ __forceinline__ uint32_t umma_ts4_probe(uint32_t d_tmem, uint32_t a_t
       "add.u32 a1, %2, 8;\n\t"
       "add.u32 a2, %2, 16;\n\t"
       "add.u32 a3, %2, 24;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%1], [%2], %3, %4, pa;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%1], [a1], d1, %4, pt;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%1], [a2], d2, %4, pt;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%1], [a3], d3, %4, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%1], [%2], %3, %4, pa;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%1], [a1], d1, %4, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%1], [a2], d2, %4, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%1], [a3], d3, %4, pt;\n\t"
+      "vote.sync.all.pred pw, pw, 0xffffffff;\n\t"
       "selp.u32 %0, 1, 0, pw;\n\t"
       "}"
       : "=r"(ready)
@@ -213,9 +254,10 @@ __device__ __forceinline__ void umma_ts4_ss8_probe2(uint32_t d_o, uint32_t a_tme
                                                     uint32_t& ready1, uint32_t& ready2) {
   asm volatile(
       "{\n\t"
-      ".reg .pred pw1, pw2, pt, pf;\n\t"
+      ".reg .pred pe, pw1, pw2, pt, pf;\n\t"
       ".reg .b64 d1, d2, d3, q1, k1;\n\t"
       ".reg .b32 a1, a2, a3;\n\t"
+      "elect.sync _|pe, 0xffffffff;\n\t"
       "mbarrier.test_wait.parity.shared::cta.b64 pw1, [%10], %11;\n\t"
       "mbarrier.test_wait.parity.shared::cta.b64 pw2, [%12], %13;\n\t"
       "setp.eq.b32 pt, 0, 0;\n\t"
@@ -226,32 +268,34 @@ __device__ __forceinline__ void umma_ts4_ss8_probe2(uint32_t d_o, uint32_t a_tme
       "add.u32 a1, %3, 8;\n\t"
       "add.u32 a2, %3, 16;\n\t"
       "add.u32 a3, %3, 24;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%2], [%3], %4, %5, pt;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%2], [a1], d1, %5, pt;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%2], [a2], d2, %5, pt;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%2], [a3], d3, %5, pt;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%6], %7, %8, %9, pf;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%2], [%3], %4, %5, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%2], [a1], d1, %5, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%2], [a2], d2, %5, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%2], [a3], d3, %5, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%6], %7, %8, %9, pf;\n\t"
       "add.u64 q1, %7, 2;\n\t"
       "add.u64 k1, %8, 2;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
       "add.u64 q1, %7, 4;\n\t"
       "add.u64 k1, %8, 4;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
       "add.u64 q1, %7, 6;\n\t"
       "add.u64 k1, %8, 6;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
       "add.u64 q1, %7, 1024;\n\t"
       "add.u64 k1, %8, 1024;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
       "add.u64 q1, %7, 1026;\n\t"
       "add.u64 k1, %8, 1026;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
       "add.u64 q1, %7, 1028;\n\t"
       "add.u64 k1, %8, 1028;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
       "add.u64 q1, %7, 1030;\n\t"
       "add.u64 k1, %8, 1030;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
+      "vote.sync.all.pred pw1, pw1, 0xffffffff;\n\t"
+      "vote.sync.all.pred pw2, pw2, 0xffffffff;\n\t"
       "selp.u32 %0, 1, 0, pw1;\n\t"
       "selp.u32 %1, 1, 0, pw2;\n\t"
       "}"
@@ -267,16 +311,18 @@ __device__ __forceinline__ uint32_t umma_ts2_probe(uint32_t d_tmem, uint32_t a_t
   uint32_t ready;
   asm volatile(
       "{\n\t"
-      ".reg .pred pw, pa, pt;\n\t"
+      ".reg .pred pe, pw, pa, pt;\n\t"
       ".reg .b64 d1, d2, d3;\n\t"
       ".reg .b32 a1, a2, a3;\n\t"
+      "elect.sync _|pe, 0xffffffff;\n\t"
       "mbarrier.test_wait.parity.shared::cta.b64 pw, [%6], %7;\n\t"
       "setp.ne.b32 pa, %5, 0;\n\t"
       "setp.eq.b32 pt, 0, 0;\n\t"
       "add.u64 d1, %3, 128;\n\t"
       "add.u32 a1, %2, 8;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%1], [%2], %3, %4, pa;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%1], [a1], d1, %4, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%1], [%2], %3, %4, pa;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%1], [a1], d1, %4, pt;\n\t"
+      "vote.sync.all.pred pw, pw, 0xffffffff;\n\t"
       "selp.u32 %0, 1, 0, pw;\n\t"
       "}"
       : "=r"(ready)
@@ -291,39 +337,42 @@ __device__ __forceinline__ void umma_ts2_ss8_probe2(uint32_t d_o, uint32_t a_tme
                                                     uint32_t& ready1, uint32_t& ready2) {
   asm volatile(
       "{\n\t"
-      ".reg .pred pw1, pw2, pt, pf;\n\t"
+      ".reg .pred pe, pw1, pw2, pt, pf;\n\t"
       ".reg .b64 d1, d2, d3, q1, k1;\n\t"
       ".reg .b32 a1, a2, a3;\n\t"
+      "elect.sync _|pe, 0xffffffff;\n\t"
       "mbarrier.test_wait.parity.shared::cta.b64 pw1, [%10], %11;\n\t"
       "mbarrier.test_wait.parity.shared::cta.b64 pw2, [%12], %13;\n\t"
       "setp.eq.b32 pt, 0, 0;\n\t"
       "setp.ne.b32 pf, 0, 0;\n\t"
       "add.u64 d1, %4, 128;\n\t"
       "add.u32 a1, %3, 8;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%2], [%3], %4, %5, pt;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%2], [a1], d1, %5, pt;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%6], %7, %8, %9, pf;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%2], [%3], %4, %5, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%2], [a1], d1, %5, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%6], %7, %8, %9, pf;\n\t"
       "add.u64 q1, %7, 2;\n\t"
       "add.u64 k1, %8, 2;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
       "add.u64 q1, %7, 4;\n\t"
       "add.u64 k1, %8, 4;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
       "add.u64 q1, %7, 6;\n\t"
       "add.u64 k1, %8, 6;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
       "add.u64 q1, %7, 1024;\n\t"
       "add.u64 k1, %8, 1024;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
       "add.u64 q1, %7, 1026;\n\t"
       "add.u64 k1, %8, 1026;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
       "add.u64 q1, %7, 1028;\n\t"
       "add.u64 k1, %8, 1028;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
       "add.u64 q1, %7, 1030;\n\t"
       "add.u64 k1, %8, 1030;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%6], q1, k1, %9, pt;\n\t"
+      "vote.sync.all.pred pw1, pw1, 0xffffffff;\n\t"
+      "vote.sync.all.pred pw2, pw2, 0xffffffff;\n\t"
       "selp.u32 %0, 1, 0, pw1;\n\t"
       "selp.u32 %1, 1, 0, pw2;\n\t"
       "}"
@@ -340,32 +389,35 @@ __device__ __forceinline__ void umma_ss8_probe2(uint32_t d_s, uint64_t q_desc, u
                                                 uint32_t bar2, uint32_t parity2, uint32_t& ready1, uint32_t& ready2) {
   asm volatile(
       "{\n\t"
-      ".reg .pred pw1, pw2, pt, pf;\n\t"
+      ".reg .pred pe, pw1, pw2, pt, pf;\n\t"
       ".reg .b64 q1, k1;\n\t"
+      "elect.sync _|pe, 0xffffffff;\n\t"
       "mbarrier.test_wait.parity.shared::cta.b64 pw1, [%6], %7;\n\t"
       "mbarrier.test_wait.parity.shared::cta.b64 pw2, [%8], %9;\n\t"
       "setp.eq.b32 pt, 0, 0;\n\t"
       "setp.ne.b32 pf, 0, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%2], %3, %4, %5, pf;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%2], %3, %4, %5, pf;\n\t"
       "add.u64 q1, %3, 2;\n\t"
       "add.u64 k1, %4, 2;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%2], q1, k1, %5, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%2], q1, k1, %5, pt;\n\t"
       "add.u64 q1, %3, 4;\n\t"
       "add.u64 k1, %4, 4;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%2], q1, k1, %5, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%2], q1, k1, %5, pt;\n\t"
       "add.u64 q1, %3, 6;\n\t"
       "add.u64 k1, %4, 6;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%2], q1, k1, %5, pt;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%2], %10, %11, %5, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%2], q1, k1, %5, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%2], %10, %11, %5, pt;\n\t"
       "add.u64 q1, %10, 2;\n\t"
       "add.u64 k1, %11, 2;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%2], q1, k1, %5, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%2], q1, k1, %5, pt;\n\t"
       "add.u64 q1, %10, 4;\n\t"
       "add.u64 k1, %11, 4;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%2], q1, k1, %5, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%2], q1, k1, %5, pt;\n\t"
       "add.u64 q1, %10, 6;\n\t"
       "add.u64 k1, %11, 6;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%2], q1, k1, %5, pt;\n\t"
+      "@pe tcgen05.mma.cta_group::1.kind::f16 [%2], q1, k1, %5, pt;\n\t"
+      "vote.sync.all.pred pw1, pw1, 0xffffffff;\n\t"
+      "vote.sync.all.pred pw2, pw2, 0xffffffff;\n\t"
       "selp.u32 %0, 1, 0, pw1;\n\t"
       "selp.u32 %1, 1, 0, pw2;\n\t"
       "}"
