@@ -78,6 +78,12 @@ __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile
   return mbar_wait_bounded(bar, parity, abort_flag, status, kStLinear, kWaitLimitNs);
 }
 
+// The same for a whole converged warp.
+__device__ __forceinline__ bool wait_bar_warp(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag,
+                                              uint32_t* status) {
+  return __all_sync(0xffffffffu, wait_bar(bar, parity, abort_flag, status));
+}
+
 // Order-preserving map float -> unsigned (0 lies below every float), so that a row maximum can be
 // taken with atomicMax, which does not depend on the order of the updates.
 __device__ __forceinline__ uint32_t float_key(float x) {
@@ -106,7 +112,7 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
   volatile uint32_t* abort_flag = flags;
   auto bar = [&](int i) -> uint32_t { return base + kOffBar + 8u * static_cast<uint32_t>(i); };
 
-  const int warp = threadIdx.x >> 5;
+  const int warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);  // known to be the same in the warp
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_cta_rank();  // 0: issues the pair's MMAs
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
@@ -151,7 +157,7 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
   cluster_arrive();
   cluster_wait();
   tc_fence_after();
-  const uint32_t tmem_base = flags[1];
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, flags[1], 0);
   grid_dependency_wait();
   // The kernel behind a projection may set itself up on SMs that run out of work (sub-block at 512 pixels 141.2 us
   // without, 138.9 with). Not between the wide attention's launches (4096 x 512: 61.4 us without, 62.7 with).
@@ -208,16 +214,18 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
     __syncwarp();
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0 && rank == 0) {
+    // The whole warp, with an elected lane (see umma_ts_warp): sub-block at 512 pixels 141.6 -> 139.6 us, wide attention
+    // 4096 x 512 60.4 -> 59.5, 16384 x 512 634 -> 623. (A second warp for the loads of W: no difference.)
+    if (rank == 0) {
       constexpr uint32_t idesc = umma_idesc_f16(2 * kTM, kTN, 0, 0);
       uint32_t it = 0;
       int local = 0;
-      bool ok = *abort_flag == 0u;
+      bool ok = __all_sync(0xffffffffu, *abort_flag == 0u);
       for (int item = pair; item < n_items && ok; item += n_pairs, ++local) {
         const int b = local & 1;
         const uint32_t use = static_cast<uint32_t>(local >> 1);
         // The epilogue warps must have drained this accumulator (first use passes at once).
-        ok = wait_bar(bar(kBarAccEmpty + b), (use & 1u) ^ 1u, abort_flag, a.status);
+        ok = wait_bar_warp(bar(kBarAccEmpty + b), (use & 1u) ^ 1u, abort_flag, a.status);
         if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + 256u * b;
@@ -225,7 +233,7 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
         for (int ks = k_first, ke = end_k(item); ks < ke; ++ks, ++it) {
           const uint32_t stage = it % kStages;
           const uint32_t phase = (it / kStages) & 1u;
-          ok = wait_bar(bar(kBarFull + stage), phase, abort_flag, a.status);
+          ok = wait_bar_warp(bar(kBarFull + stage), phase, abort_flag, a.status);
           if (!ok) break;
           const uint32_t a_addr = base + stage * kStageBytes;
           const uint64_t desc_a = smem_desc_sw128(a_addr, 16, 1024);
@@ -233,16 +241,16 @@ linear_kernel(const __grid_constant__ LinearMaps maps, const LinearArgs a) {
           // Four MMAs per stage, each 32 bytes (K = 16 halves) further along the swizzled rows.
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk)
-            umma_ss_pair(d_tmem, desc_a + 2u * kk, desc_b + 2u * kk, idesc, (ks > k_first || kk > 0) ? 1u : 0u);
-          umma_commit_pair(bar(kBarEmpty + stage), 3);  // both CTAs' producers may refill the stage
+            umma_ss_pair_warp(d_tmem, desc_a + 2u * kk, desc_b + 2u * kk, idesc, (ks > k_first || kk > 0) ? 1u : 0u);
+          umma_commit_pair_warp(bar(kBarEmpty + stage), 3);  // both CTAs' producers may refill the stage
         }
         if (!ok) break;
-        umma_commit_pair(bar(kBarAccFull + b), 3);  // both CTAs' epilogues may read their rows
+        umma_commit_pair_warp(bar(kBarAccFull + b), 3);  // both CTAs' epilogues may read their rows
       }
       if (!ok) {
-        umma_commit_pair(bar(kBarDrain), 1);
+        umma_commit_pair_warp(bar(kBarDrain), 1);
         const uint64_t t0 = globaltimer_ns();
-        while (!mbar_try_wait(bar(kBarDrain), 0) && globaltimer_ns() - t0 < kWaitLimitNs) {
+        while (!__all_sync(0xffffffffu, mbar_try_wait(bar(kBarDrain), 0) || globaltimer_ns() - t0 >= kWaitLimitNs)) {
         }
       }
     }
