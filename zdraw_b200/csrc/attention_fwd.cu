@@ -220,6 +220,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, flags[1], 0);
 
+  if (threadIdx.x == 0) {  // launch parameters: no earlier kernel writes them (80 x 2 in f32 9.29 -> 9.15 us, 1536 x 24 38.54 -> 38.40)
+    tma_prefetch_desc(&tm_q);
+    tma_prefetch_desc(&tm_k);
+    tma_prefetch_desc(&tm_v);
+  }
   // Everything above overlaps the tail of the preceding kernel (the prologue) when the launch
   // allows it; from here on this kernel reads what earlier kernels wrote.
   grid_dependency_wait();
@@ -243,9 +248,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
     if (warp == 0) {
       // ---------------------------------------------------------- TMA producer
       if (lane == 0 && n_act > 0) {
-        tma_prefetch_desc(&tm_q);
-        tma_prefetch_desc(&tm_k);
-        tma_prefetch_desc(&tm_v);
         for (int t = 0; t < 2; ++t) {
           const int row = (q_tile0 + t) * kBM;
           const uint32_t dst = base + kOffQ + t * kTileBytes;
@@ -807,6 +809,11 @@ attn_fwd_steps_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, flags[1], 0);
+  if (threadIdx.x == 0) {
+    tma_prefetch_desc(&tm_q);
+    tma_prefetch_desc(&tm_k);
+    tma_prefetch_desc(&tm_v);
+  }
   grid_dependency_wait();
 
   auto c1 = [&](int hm, int tok) { return hm ? tok : head; };
@@ -820,9 +827,6 @@ attn_fwd_steps_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     if (warp == 0) {
       // ---------------------------------------------------------- TMA producer
       if (lane == 0 && n_act > 0) {
-        tma_prefetch_desc(&tm_q);
-        tma_prefetch_desc(&tm_k);
-        tma_prefetch_desc(&tm_v);
         {
           const int row = q_tile * kBM;
           mbar_arrive_expect_tx(bar(kS1BarQFull), kTileBytes);
