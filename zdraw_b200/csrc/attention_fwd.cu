@@ -1343,7 +1343,7 @@ cudaError_t attn_fwd_configure() {
 bool attn_fwd_takes_steps_kernel(int tokens, int heads, int batch, int sm_count, bool traced) {
   // When every query tile can have an SM of its own, one tile per CTA with its K/V steps
   // interleaved finishes sooner: a two-tile CTA's time is set by one tile's chain, not by how many
-  // tiles it holds (klein_1024 with 3 heads, 108 tiles: 41 us against 60). With more tiles than SMs
+  // tiles it holds (4608 tokens x 3 heads, 108 tiles: 41 us against 60, now 37). With more tiles than SMs
   // the two-tile kernel's single wave wins again (6 heads, 216 tiles: 81 us against 61).
   const long long n_q_tiles = (tokens + kBM - 1) / kBM;
   return !traced && sm_count > 0 && n_q_tiles * heads * batch <= sm_count;

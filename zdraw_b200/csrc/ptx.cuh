@@ -526,28 +526,7 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols
 }
 // D[tmem of both CTAs] (+)= A * B with M = 256 over the pair: rows [0,128) of A and D belong to
 // the issuing (even-rank) CTA, rows [128,256) to its peer; each CTA holds half of B's N rows. The
-// descriptors are offsets valid in both CTAs' shared memory.
-__device__ __forceinline__ void umma_ss_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                             uint32_t accumulate) {
-  asm volatile(
-      "{\n\t"
-      ".reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t"
-      "}" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// When every MMA issued so far has finished, arrive once on the mbarrier at this shared-memory
-// offset in each CTA named by cta_mask.
-__device__ __forceinline__ void umma_commit_pair(uint32_t bar, uint16_t cta_mask) {
-  asm volatile(
-      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
-      "h"(cta_mask)
-      : "memory");
-}
-
-// The same from a whole converged warp (see umma_ts_warp).
+// descriptors are offsets valid in both CTAs' shared memory. From a whole converged warp (see umma_ts_warp).
 __device__ __forceinline__ void umma_ss_pair_warp(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                                   uint32_t accumulate) {
   asm volatile(
@@ -560,6 +539,8 @@ __device__ __forceinline__ void umma_ss_pair_warp(uint32_t d_tmem, uint64_t a_de
       "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// When every MMA issued so far has finished, arrive once on the mbarrier at this shared-memory
+// offset in each CTA named by cta_mask.
 __device__ __forceinline__ void umma_commit_pair_warp(uint32_t bar, uint16_t cta_mask) {
   asm volatile(
       "{\n\t"
