@@ -220,7 +220,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant_
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, flags[1], 0);
 
-  if (threadIdx.x == 0) {  // launch parameters: no earlier kernel writes them (80 x 2 in f32 9.29 -> 9.15 us, 1536 x 24 38.54 -> 38.40)
+  if (threadIdx.x == 0) {  // launch parameters: no earlier kernel writes them (1536 x 24 38.54 -> 38.40 us)
     tma_prefetch_desc(&tm_q);
     tma_prefetch_desc(&tm_k);
     tma_prefetch_desc(&tm_v);
